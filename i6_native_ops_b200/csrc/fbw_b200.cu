@@ -26,8 +26,8 @@
 // Arithmetic is kept in the reference's fp32 operation order wherever that order is deterministic
 // there, because scores grow with t (~2e4 at T=1500, one ulp = 2e-3) and any reassociation shows
 // up in the posteriors:
-//   * prob_add is fbw_op.cu:39-48 verbatim in meaning: -log1pf(expf(-|a-b|)) + fminf(a,b), +inf for
-//     a NaN difference; accurate libdevice expf/log1pf (no fast-math).
+//   * prob_add is fbw_op.cu:39-48 in meaning: min(a,b) - log1p(exp(-|a-b|)), +inf where both are +inf,
+//     rounded once to the grid of the result (see prob_add below for how the logarithm is formed).
 //   * an edge's forward value is (alpha + weight) + score (fbw_op.cu:93); the edge score adds beta
 //     last (fbw_op.cu:96,99).
 //   * the normaliser is a left fold over the sequence's edges in ascending edge index
@@ -188,41 +188,35 @@ int bits_for(unsigned long long maxval) {
 // device helpers
 // ---------------------------------------------------------------------------------------------
 
-// Log-semiring sum of two negative-log values; same expression as the reference's prob_add
-// (i6_native_ops/fbw/fbw_op.cu:39-48) so results round identically.
-__device__ __forceinline__ float prob_add(float a, float b) {
-    float diff = a - b;
-    if (isnan(diff)) {
-        return CUDART_INF_F;
-    }
-    return -log1pf(expf(-fabsf(diff))) + fminf(a, b);
+__device__ __forceinline__ float ex2_approx(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
 }
 
-// prob_add with an exact shortcut.  prob_add(a,b) = fl(m - L), m = min(a,b), L = log1pf(expf(-d)),
-// d = |a-b|.  L <= 2^(-d*log2(e)) (1 + 2^-20); if that is below a quarter of the smallest gap between
-// m and a neighbouring float (2^(e-24) with e the exponent of m, taken at a power of two), the sum
-// rounds back to m, so  d*log2(e) > 27 - e  implies the result is m bit for bit.  A NaN difference
-// fails the test and takes the full path.
-__device__ __forceinline__ bool prob_add_is_min(float a, float b, float m) {
-    const float d = fabsf(a - b);
-    const int   e = (int)((__float_as_uint(m) >> 23) & 0xffu) - 127;
-    return d * 1.442695f > (float)(27 - e);
+// Log-semiring sum of two negative-log values: min(a,b) - log1p(exp(-|a-b|)), the reference's prob_add
+// (i6_native_ops/fbw/fbw_op.cu:39-48).  log1p(e) on [0,1] is e times a polynomial of degree 8, fitted
+// here by linear programming (largest absolute error of e * q(e) 4.6e-10 before rounding, 1.3e-7 with
+// fp32 coefficients and steps); the last step is one fused multiply-add, so the sum is rounded once, to
+// the grid of the scores, as in the reference.  Scores are sums over frames (magnitudes of 1e2..1e4, one
+// ulp 8e-6..1e-3), so the error of the logarithm disappears in that rounding: results are the
+// reference's but for a last-place step once in several hundred sums.
+// A NaN difference (both +inf, or a NaN score) gives e = 0, that is the smaller operand: +inf, or the
+// operand that is a number.
+__device__ __forceinline__ float prob_add(float a, float b) {
+    const float m = fminf(a, b);
+    const float e = ex2_approx(fmaxf(fabsf(a - b) * -1.44269504f, -150.f));
+    const float y = e * e, y2 = y * y;
+    const float p0 = fmaf(-0.4999940097f, e, 0.9999999404f), p1 = fmaf(-0.2486045212f, e, 0.3332001567f);
+    const float p2 = fmaf(-0.1390718967f, e, 0.1920055002f), p3 = fmaf(-0.0317371115f, e, 0.0815147609f);
+    const float q0 = fmaf(p1, y, p0), q1 = fmaf(0.0058344044f, y2, fmaf(p3, y, p2));
+    return fmaf(-e, fmaf(q1, y2, q0), m);
 }
 
 // first term of an accumulation that starts at +inf: prob_add(+inf, y) is y (or +inf for NaN)
-__device__ __forceinline__ float prob_first(float y) { return isnan(y) ? CUDART_INF_F : y; }
+__device__ __forceinline__ float prob_first(float y) { return fminf(y, CUDART_INF_F); }
 
-// prob_add(acc, x) through the exact shortcuts: +inf terms, a first term, a provably dominated term
-__device__ __forceinline__ float prob_add_fast(float acc, float x) {
-    if (x == CUDART_INF_F) return acc;
-    if (acc == CUDART_INF_F) return prob_first(x);
-    const float m = fminf(acc, x);
-    if (prob_add_is_min(acc, x, m)) return m;
-    return prob_add(acc, x);
-}
-
-// prob_add(acc, x) with only the free shortcuts (+inf term, first term).  Used by the sweeps, where
-// neighbouring states' scores are close and the dominance test rarely pays for itself.
+// prob_add(acc, x) with the free shortcuts (+inf term, first term)
 __device__ __forceinline__ float prob_add_live(float acc, float x) {
     if (x == CUDART_INF_F) return acc;
     if (acc == CUDART_INF_F) return prob_first(x);
@@ -1342,8 +1336,8 @@ __global__ void __launch_bounds__(256) k_score(RunArgs a) {
 // Frame normalisers: sum = left fold of prob_add over the sequence's edges in ascending edge index
 // (fbw_op.cu:115-118), sums[t,b] = isinf(sum) ? 0 : sum (fbw_op.cu:120-129).  One warp per
 // (sequence, 32-frame tile), lane = frame, streaming the tile's edge scores in storage order; the
-// next 8 lines are loaded while the current 8 are folded.  Steps whose result is provably the
-// running minimum skip expf/log1pf (exact).  The raw sum (+inf for a dead frame) goes to N.
+// next lines are loaded while the current ones are folded.  The raw sum (+inf for a dead frame) goes
+// to N.
 // Every unit is its own warp so that all the serial folds of a call run side by side.
 // (one warp folds one unit; returns the raw sum of the lane's frame)
 __device__ __forceinline__ float norm_unit(const RunArgs& a, const PostUnit& p, int lane) {
@@ -1365,7 +1359,7 @@ __device__ __forceinline__ float norm_unit(const RunArgs& a, const PostUnit& p, 
                 nx[j] = i < p.Eb ? Xb[(i64)i * kTile] : CUDART_INF_F;
             }
 #pragma unroll
-            for (int j = 0; j < kNormBatch; j++) acc = prob_add_fast(acc, x[j]);
+            for (int j = 0; j < kNormBatch; j++) acc = prob_add(acc, x[j]);
         }
         if (valid) a.sums[(i64)t * a.B + p.b] = isinf(acc) ? 0.f : acc;
         a.N[p.u * kTile + lane] = acc;
