@@ -10,9 +10,9 @@
 //               sequences by cost.
 //   k_gather  : am_scores[t,b,emission] for the distinct emissions of each sequence -> compact
 //               score arrays (frame-major for the sweeps, 32-frame tiles for the score pass).
-//   k_sweep   : one persistent CTA per (sequence, direction); the automaton lives in shared memory
-//               and registers, frames are stepped with one barrier each, next frames' scores arrive
-//               by cp.async; state scores leave as full 128-byte lines of a tiled layout.
+//   k_sweep,  : one persistent CTA, or cluster, per (sequence, direction); the automaton lives in shared
+//   k_sweep_small  memory and registers, frames are stepped with one barrier each, next frames' scores
+//               arrive by cp.async; state scores leave eight frames at a time (sweep_b200.inc).
 //   k_score   : time-parallel; edge scores of every (frame, edge), lane = frame.
 //   k_norm    : per (sequence, 32 frames): the frame normaliser, a serial left fold.
 //   k_class   : per (sequence, 32 frames): the class posteriors.
@@ -23,16 +23,17 @@
 // For scores and results in pinned host memory the library's host threads (host_fill.cpp) pick the
 // scores out of the tensor and write the result's rows from the posteriors the device sends.
 //
-// Arithmetic is kept in the reference's fp32 operation order wherever that order is deterministic
-// there, because scores grow with t (~2e4 at T=1500, one ulp = 2e-3) and any reassociation shows
-// up in the posteriors:
+// Arithmetic.  Scores grow with t (~2e4 at T=1500, one ulp = 2e-3), and a sum of two of them rounded to
+// that grid, as the reference forms it, shows in the posteriors:
+//   * the sweeps' log-sums are formed in scaled numbers (to_scaled): one relative rounding of 2^-24 per
+//     operation, whatever the accumulated score.  A stored state score is the natural negative log, rounded
+//     once; it is closer to the exact value than the reference's.
 //   * prob_add is fbw_op.cu:39-48 in meaning: min(a,b) - log1p(exp(-|a-b|)), +inf where both are +inf,
 //     rounded once to the grid of the result (see prob_add below for how the logarithm is formed).
-//   * an edge's forward value is (alpha + weight) + score (fbw_op.cu:93); the edge score adds beta
-//     last (fbw_op.cu:96,99).
+//   * an edge score is ((alpha + weight) + score) + beta (fbw_op.cu:93-99).
 //   * the normaliser is a left fold over the sequence's edges in ascending edge index
-//     (fbw_op.cu:115-118); state and class accumulations also run in ascending edge index (the
-//     reference's atomics have no defined order; with at most two terms the order is immaterial).
+//     (fbw_op.cu:115-118); class accumulations also run in ascending edge index (the reference's
+//     atomics have no defined order; with at most two terms the order is immaterial).
 
 #include "fbw_b200.h"
 #include "host_fill.h"
@@ -221,6 +222,41 @@ __device__ __forceinline__ float prob_add_live(float acc, float x) {
     if (x == CUDART_INF_F) return acc;
     if (acc == CUDART_INF_F) return prob_first(x);
     return prob_add(acc, x);
+}
+
+// Scaled numbers: x.x * 2^-x.y with x.y a whole number, +inf for zero (a dead state or edge).  The
+// exponent is a float so that +inf needs no special case and scores of any magnitude fit (above 2^24 its
+// spacing exceeds one, as the spacing of a score of that magnitude does).
+//
+// exp(-s) of a negative log score: s * log2(e) is split into the nearest whole number and a remainder,
+// formed with fused multiply-adds and log2(e) in two parts, so the mantissa (0.70 .. 1.42) carries the
+// score's own rounding and the exponential's (2^-22.5) only.  +inf and NaN give zero; finite scores beyond
+// the exponent's range saturate and stay finite.
+__device__ __forceinline__ float2 to_scaled(float s) {
+    const float c = rintf(fminf(fmaxf(s * 1.44269502f, -3.4e38f), 3.4e38f));
+    float r = fmaf(s, 1.44269502f, -c);
+    r = fmaf(s, 1.92596303e-8f, r);
+    r = fminf(fmaxf(r, -0.75f), 0.75f);
+    return make_float2(ex2_approx(-r), s < CUDART_INF_F ? c : CUDART_INF_F);
+}
+
+// 2^d for a whole number d <= 0; zero below 2^-126 and for NaN (the difference of two +inf)
+__device__ __forceinline__ float pow2_neg(float d) {
+    return __uint_as_float(__float_as_uint(fmaxf(d, -127.f) + 8388735.f) << 23);
+}
+
+// acc * 2^-c with the mantissa brought into [1,2); acc = 0 only where c = +inf
+__device__ __forceinline__ float2 normalised(float acc, float c) {
+    const unsigned u = __float_as_uint(acc);
+    return make_float2(__uint_as_float((u & 0x007fffffu) | 0x3f800000u),
+                       c - (__uint_as_float(0x4b000000u | (u >> 23)) - 8388735.f));
+}
+
+// the natural negative log of a scaled number (mantissa in [1,2)), rounded once
+__device__ __forceinline__ float from_scaled(float2 x) {
+    float l;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(x.x));
+    return x.y < 3.4e38f ? fmaf(x.y, 0.693147181f, l * -0.693147181f) : x.y;
 }
 
 // largest b in [0,B) with off[b] <= u, given off[0] <= u < off[B]
@@ -815,6 +851,7 @@ struct RunArgs {
     float*       sums;
     float*       loss2;
     float *A, *Bt, *Gt, *Gf, *P, *X, *N;
+    float2* Gs;    // gathered scores as scaled numbers, frame-major (k_sweep_small); null: raw scores to Gf
     const int *state_off, *edge_off, *slot_off, *nslot, *seq_T, *start_l, *end_l;
     const i64 *ta_off, *tg_off, *gf_off, *gu_off, *pu_off, *tx_off;
     const int2* m_pos;
@@ -827,7 +864,7 @@ struct RunArgs {
     // Time chunks: the sweeps advance chunk_steps frames per chunk from both ends of a sequence; a
     // launch handles the chunks [c_lo, c_hi).  One chunk covering everything is the plain case.
     int c_lo, c_hi, chunk_steps;
-    float* carry;  // state vectors handed from one sweep chunk to the next, [2 * state][direction]
+    float* carry;  // state vectors handed from one sweep chunk to the next, float or float2 [2 * state][direction]
     // 1: the wrapper's passes are folded in -- `am` is log_probs (B,T,F) (sign and layout of the
     // caller's tensor, i6_native_ops/fbw/__init__.py:66) and `out` receives the gradient with respect
     // to it, -posterior in (B,T,F) with zeros elsewhere (what __init__.py:41-44 and autograd produce)
@@ -869,7 +906,8 @@ __device__ __forceinline__ bool in_chunks(int c, const RunArgs& a) { return c >=
 
 // Gather am_scores[t,b,emission] for the distinct emissions ("slots", ascending emission id) of
 // each sequence.  Work item = (sequence, 32-frame tile, 256 slots).  Two copies are written:
-//   Gf  frame-major  [t][slot]           (rows padded to 4 floats)  -- read by the sweeps
+//   Gf  frame-major  [t][slot]           (rows padded to 4 floats)  -- read by the sweeps, or instead
+//   Gs  the same as scaled numbers                                  -- read by k_sweep_small
 //   Gt  tiled        [t/32][slot][t%32]                              -- read by k_post, lane = frame
 __global__ void __launch_bounds__(256) k_gather(RunArgs a) {
     __shared__ float tile[kTile][kGatherSlots + 1];
@@ -891,6 +929,7 @@ __global__ void __launch_bounds__(256) k_gather(RunArgs a) {
         const int nd = min(kGatherSlots, Db - d0);
         const int* __restrict__ emis = a.slot_emis + so + d0;
         float* __restrict__ gf = a.Gf + a.gf_off[b];
+        float2* __restrict__ gs = a.Gs ? a.Gs + a.gf_off[b] : nullptr;
         float* __restrict__ gt = a.Gt ? a.Gt + a.tg_off[b] + ((i64)k * Db + d0) * kTile : nullptr;
 
         int em[kGatherSlots / 32];
@@ -918,11 +957,15 @@ __global__ void __launch_bounds__(256) k_gather(RunArgs a) {
                 int dd = lane + 32 * j;
                 if (dd < nd) {
                     tile[f][dd] = v[j];
-                    if (valid && !a.gathered_by_host) gf[(i64)t * Dp + d0 + dd] = v[j];
+                    if (valid && gs) gs[(i64)t * Dp + d0 + dd] = to_scaled(v[j]);
+                    if (valid && !gs && !a.gathered_by_host) gf[(i64)t * Dp + d0 + dd] = v[j];
                 }
             }
-            if (valid && c == nch - 1 && !a.gathered_by_host) {
-                for (int dd = Db + lane; dd < Dp; dd += 32) gf[(i64)t * Dp + dd] = 0.f;
+            if (valid && c == nch - 1) {
+                for (int dd = Db + lane; dd < Dp; dd += 32) {
+                    if (gs) gs[(i64)t * Dp + dd] = make_float2(1.f, CUDART_INF_F);
+                    else if (!a.gathered_by_host) gf[(i64)t * Dp + dd] = 0.f;
+                }
             }
         }
         __syncthreads();
@@ -1692,7 +1735,7 @@ __global__ void __launch_bounds__(1024) k_loss(const float* __restrict__ sums, i
 // host side
 // ---------------------------------------------------------------------------------------------
 struct RunLayout {
-    size_t A, Bt, Gt, Gf, P, X, N, carry, next_row, total;
+    size_t A, Bt, Gt, Gf, Gs, P, X, N, carry, next_row, total;
 };
 
 RunLayout run_layout(const fbw_b200_summary& s) {
@@ -1707,10 +1750,11 @@ RunLayout run_layout(const fbw_b200_summary& s) {
     L.Bt    = take((size_t)s.state_floats);
     L.Gt    = take((size_t)s.tiled_floats);
     L.Gf    = take((size_t)s.frame_floats);
+    L.Gs    = take((size_t)s.frame_floats * 2);
     L.P     = take((size_t)s.frame_floats);
     L.X     = take((size_t)s.score_floats);
     L.N     = take((size_t)s.post_units * kTile);
-    L.carry = take((size_t)(2 * s.S));
+    L.carry = take((size_t)(4 * s.S));
     L.next_row = take(2 * FBW_B200_GROUPS);  // a 64-bit row counter per group (background_rows)
     L.total = off;
     return L;
@@ -1786,6 +1830,7 @@ RunArgs fbw_args(const void* plan, const fbw_b200_summary& s, void* work, const 
     a.Bt = at<float>(work, R.Bt);
     a.Gt = at<float>(work, R.Gt);
     a.Gf = at<float>(work, R.Gf);
+    a.Gs = at<float2>(work, R.Gs);
     a.P  = at<float>(work, R.P);
     a.X  = at<float>(work, R.X);
     a.N  = at<float>(work, R.N);
@@ -1874,11 +1919,13 @@ int launch_sweep(const RunArgs& a, int grid, int nt, size_t smem, int smax, int 
 }
 
 #include "sweep_cluster_b200.inc"
+#include "sweep_scaled_b200.inc"
+
 // CTAs per cluster for the sweeps of `items` (sequence, direction) pairs of automata of at most ms
 // states, when `spare` SMs would otherwise stay idle during the call's sweeps.  A cluster spreads the
 // per-frame work of one large sequence over several SMs, which shortens the call only while SMs are
 // free: a call that already has a sweep CTA for every SM gains nothing and pays for the cluster
-// barriers.  Returns 1, 2 or 4 and takes the SMs it uses off `spare`.  FBW_B200_CLUSTER=1|2|4 fixes
+// barriers.  Returns 1, 2, 4 or 8 and takes the SMs it uses off `spare`.  FBW_B200_CLUSTER=1|2|4|8 fixes
 // the answer.
 int sweep_cluster_size(i64 ms, int items, int* spare) {
     static int forced = -1;
@@ -1886,9 +1933,10 @@ int sweep_cluster_size(i64 ms, int items, int* spare) {
         const char* e = getenv("FBW_B200_CLUSTER");
         forced = e ? atoi(e) : 0;
     }
-    if (forced == 1 || forced == 2 || forced == 4) return forced;
+    if (forced == 1 || forced == 2 || forced == 4 || forced == 8) return forced;
     if (ms <= 1024 || items <= 0) return 1;
-    for (int cs = ms > 2048 ? 4 : 2; cs > 1; cs >>= 1) {
+    // (8 lattice sequences, ms a training step: clusters of two 5.7, of four 4.2, of eight 3.4)
+    for (int cs = ms > 2048 ? 8 : 4; cs > 1; cs >>= 1) {
         const int extra = (cs - 1) * items;
         if (extra <= *spare) {
             *spare -= extra;
@@ -2054,8 +2102,9 @@ bool output_in_two_steps(const fbw_b200_summary& s, i64 ms, i64 me, i64 md) {
     if (!c.found) return false;
     if (conf == 1) return true;
     if (md * 16 > s.F) return false;  // dense rows: patching would touch most sectors twice
-    const i64 by_smem    = (i64)(227 * 1024) / (i64)(c.smem + sizeof(float) * 512 + 128 + 1024);
-    const i64 by_threads = 2048 / (c.nt + 32);
+    const ScaledShape sc = scaled_shape(ms, me, md, s.max_degree, 1);
+    const i64 by_smem    = (i64)(227 * 1024) / (i64)((sc.found ? sc.smem : c.smem) + sizeof(float) * 512 + 128 + 1024);
+    const i64 by_threads = sc.found ? 1024 / (sc.nt + 32) : 2048 / (c.nt + 32);  // (64 registers a thread)
     const i64 per_sm     = by_smem < by_threads ? (by_smem > 0 ? by_smem : 1) : (by_threads > 0 ? by_threads : 1);
     const i64 waves      = (2 * s.B + per_sm * sm_count() - 1) / (per_sm * sm_count());
     if (waves <= 1) return true;
@@ -2076,6 +2125,8 @@ int launch_group(RunArgs a, int r0, int r1, i64 ms, i64 me, i64 md, const fbw_b2
     a.r0 = r0;
     a.r1 = r1;
     const i64 tiles = (s.max_len + kTile - 1) / kTile;
+    const ScaledShape sc = scaled_shape(ms, me, md, s.max_degree, cs);
+    if (!sc.found || cs > 1) a.Gs = nullptr;  // those sweeps read the raw scores
     if (ev) CUDA_OK(cudaEventRecord(ev[0], st));
     if ((what & kDoGather) && s.gather_units > 0 && md > 0) {
         i64 want = tiles * nb * ((md + kGatherSlots - 1) / kGatherSlots);
@@ -2084,8 +2135,24 @@ int launch_group(RunArgs a, int r0, int r1, i64 ms, i64 me, i64 md, const fbw_b2
         COUNT_LAUNCH(1);
     }
     if (ev) CUDA_OK(cudaEventRecord(ev[1], st));
-    if ((what & kDoSweep) && s.max_len > 0 && cs > 1 && cluster_shape(ms, me, md, cs).found) {
-        const int rc = launch_sweepc(a, cluster_shape(ms, me, md, cs), 2 * nb, st);
+    if ((what & kDoSweep) && s.max_len > 0 && sc.found) {
+        int rc;
+        if (cs > 1) {
+            rc = launch_cluster(a, sc, 2 * nb, st);
+        } else {
+            // with the background: its block behind the sweep's shared memory, a warp more per CTA, and
+            // CTAs that do nothing else
+            size_t smem = sc.smem;
+            if (a.next_row != nullptr) {
+                a.fill_offset = (int)((sc.smem + 127) & ~(size_t)127);
+                smem = (size_t)a.fill_offset + sizeof(float) * (size_t)a.fill_piece;
+            }
+            rc = launch_small(a, sc, 2 * nb + (a.next_row != nullptr ? a.fill_ctas : 0),
+                              sc.nt + (a.next_row != nullptr ? 32 : 0), smem, st);
+        }
+        if (rc != FBW_B200_OK) return rc;
+    } else if ((what & kDoSweep) && s.max_len > 0 && cs > 1 && cluster_shape(ms, me, md, cs < 4 ? cs : 4).found) {
+        const int rc = launch_sweepc(a, cluster_shape(ms, me, md, cs < 4 ? cs : 4), 2 * nb, st);
         if (rc != FBW_B200_OK) return rc;
     } else if ((what & kDoSweep) && s.max_len > 0) {
         const SweepShape c = sweep_shape(ms, me, md);
