@@ -13,9 +13,8 @@
 //   k_sweep,  : one persistent CTA, or cluster, per (sequence, direction); the automaton lives in shared
 //   k_sweep_small  memory and registers, frames are stepped with one barrier each, next frames' scores
 //               arrive by cp.async; state scores leave eight frames at a time (sweep_b200.inc).
-//   k_score   : time-parallel; edge scores of every (frame, edge), lane = frame.
-//   k_norm    : per (sequence, 32 frames): the frame normaliser, a serial left fold.
-//   k_class   : per (sequence, 32 frames): the class posteriors.
+//   k_post    : per (sequence, 32 frames), lane = frame: edge scores, frame normalisers and class
+//               posteriors, none of which but the posteriors goes through memory.
 //   k_expand  : streams the (T,B,F) output: +inf rows with the few finite posteriors patched in.
 //   k_patch   : large calls with sparse rows write the output in two steps instead: a warp more per
 //               sweep CTA writes the +inf background through the copy engine while the sweeps run
@@ -31,9 +30,9 @@
 //   * prob_add is fbw_op.cu:39-48 in meaning: min(a,b) - log1p(exp(-|a-b|)), +inf where both are +inf,
 //     rounded once to the grid of the result (see prob_add below for how the logarithm is formed).
 //   * an edge score is ((alpha + weight) + score) + beta (fbw_op.cu:93-99).
-//   * the normaliser is a left fold over the sequence's edges in ascending edge index
-//     (fbw_op.cu:115-118); class accumulations also run in ascending edge index (the reference's
-//     atomics have no defined order; with at most two terms the order is immaterial).
+//   * class sums and the frame normaliser are scaled sums (minimum, sum of exp(minimum - x)) that stay
+//     differences until the end; the normaliser of sequences with few edges is the reference's left fold
+//     in ascending edge index (fbw_op.cu:115-118; see k_post).
 
 #include "fbw_b200.h"
 #include "host_fill.h"
@@ -70,13 +69,13 @@ struct PlanLayout {
     size_t ta_off, tg_off, gf_off, gu_off, pu_off;                               // i64[B+1]
     size_t order, cost;                                                          // int[B], i64[B]
     size_t tx_off;                                                               // i64[B+1]
-    size_t qpos, m_pos;                                                          // int[E], int2[E]
+    size_t qpos;                                                                 // int[E]
     size_t eiota, keyq, keyf, keyb, key32_out, qe, fe, be, me, slot_of_edge;     // [E]
     size_t key64, key64_out;                                                     // u64[E]
     size_t head, hs, m_ptr;                                                      // int[E+1]
     size_t rowcnt_f, rowptr_f, rowcnt_b, rowptr_b;                               // int[S+1]
     size_t fwd_rec, bwd_rec;                                                     // uint2[E]
-    size_t q_rec;                                                                // int4[E]
+    size_t m_rec;                                                                // int4[E]
     size_t slot_emis;                                                            // int[E]
     size_t cub_temp, cub_temp_bytes;
     size_t total;
@@ -140,7 +139,6 @@ PlanLayout plan_layout(i64 B, i64 E, i64 S) {
     L.cost         = take(8 * nB);
     L.tx_off       = take(8 * (nB + 1));
     L.qpos         = take(4 * nE);
-    L.m_pos        = take(8 * nE);
     L.eiota        = take(4 * nE);
     L.keyq         = take(4 * nE);
     L.keyf         = take(4 * nE);
@@ -162,7 +160,7 @@ PlanLayout plan_layout(i64 B, i64 E, i64 S) {
     L.rowptr_b     = take(4 * (nS + 1));
     L.fwd_rec      = take(8 * nE);
     L.bwd_rec      = take(8 * nE);
-    L.q_rec        = take(16 * nE);
+    L.m_rec        = take(16 * nE);
     L.slot_emis    = take(4 * (nE + nB + 1));
     L.cub_temp_bytes = cub_temp_need(E, S);
     L.cub_temp       = take(L.cub_temp_bytes);
@@ -683,7 +681,7 @@ __global__ void __launch_bounds__(kFastThreads) k_seqsort(
     const int* __restrict__ edges, const float* __restrict__ weights, i64 E, i64 F,
     const int* __restrict__ qe, const int* __restrict__ edge_off, const int* __restrict__ state_off,
     const int* __restrict__ packed_of, int* rowptr_f, int* rowptr_b, uint2* fwd_rec, uint2* bwd_rec,
-    int4* q_rec, int2* m_pos, int* m_ptr, int* slot_emis, int* slot_off, int* nslot,
+    int4* m_rec, int* m_ptr, int* slot_emis, int* slot_off, int* nslot,
     fbw_b200_summary* hdr) {
     extern __shared__ __align__(16) unsigned char fast_raw[];
     FastSmem& sm = *reinterpret_cast<FastSmem*>(fast_raw);
@@ -744,7 +742,7 @@ __global__ void __launch_bounds__(kFastThreads) k_seqsort(
             }
             const int i = (int)(keys[k] & pos_mask);
             sm.slot[i] = (unsigned short)slot;
-            m_pos[e0 + j] = make_int2(i, slot);
+            m_rec[e0 + j] = make_int4((int)(sm.from[i] | ((unsigned)sm.to[i] << 16)), i, slot, __float_as_int(weights[qe[e0 + i]]));
         }
     }
     if (tid == 0) {
@@ -801,10 +799,6 @@ __global__ void __launch_bounds__(kFastThreads) k_seqsort(
         if (dmax > 0) atomicMax(&sm.deg_max, dmax);
         __syncthreads();
     }
-    for (int i = tid; i < Eb; i += kFastThreads) {
-        q_rec[e0 + i] = make_int4((int)sm.from[i], (int)sm.to[i], (int)sm.slot[i],
-                                  __float_as_int(weights[qe[e0 + i]]));
-    }
     if (tid == 0 && sm.deg_max > 0) {
         atomicMax((unsigned long long*)&hdr->max_degree, (unsigned long long)sm.deg_max);
     }
@@ -814,10 +808,9 @@ __global__ void __launch_bounds__(kFastThreads) k_seqsort(
 __global__ void k_records(const int* __restrict__ edges, const float* __restrict__ weights, i64 E,
                           const int* __restrict__ packed_of, const int* __restrict__ state_off,
                           const int* __restrict__ slot_off, const int* __restrict__ slot_of_edge,
-                          const int* __restrict__ qe, const int* __restrict__ fe,
-                          const int* __restrict__ be, const int* __restrict__ me,
-                          const int* __restrict__ qpos, const int* __restrict__ edge_off,
-                          uint2* fwd_rec, uint2* bwd_rec, int4* q_rec, int2* m_pos,
+                          const int* __restrict__ fe, const int* __restrict__ be,
+                          const int* __restrict__ me, const int* __restrict__ qpos, const int* __restrict__ edge_off,
+                          uint2* fwd_rec, uint2* bwd_rec, int4* m_rec,
                           const fbw_b200_summary* hdr) {
     if (hdr->error) return;
     i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x;
@@ -835,11 +828,8 @@ __global__ void k_records(const int* __restrict__ edges, const float* __restrict
     fwd_rec[i] = make_uint2((unsigned)fr | ((unsigned)sl << 16), __float_as_uint(w));
     rec(be[i], fr, to, sl, w);
     bwd_rec[i] = make_uint2((unsigned)to | ((unsigned)sl << 16), __float_as_uint(w));
-    rec(qe[i], fr, to, sl, w);
-    q_rec[i] = make_int4(fr, to, sl, __float_as_int(w));
     rec(me[i], fr, to, sl, w);
-    // (position in the sequence's ascending edge list, slot) for the class-posterior pass
-    m_pos[i] = make_int2(qpos[me[i]] - edge_off[edges[3 * E + me[i]]], sl);
+    m_rec[i] = make_int4((int)((unsigned)fr | ((unsigned)to << 16)), qpos[me[i]] - edge_off[edges[3 * E + me[i]]], sl, __float_as_int(w));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -850,14 +840,13 @@ struct RunArgs {
     float*       out;
     float*       sums;
     float*       loss2;
-    float *A, *Bt, *Gt, *Gf, *P, *X, *N;
+    float *A, *Bt, *Gt, *Gf, *P;
     float2* Gs;    // gathered scores as scaled numbers, frame-major (k_sweep_small); null: raw scores to Gf
     const int *state_off, *edge_off, *slot_off, *nslot, *seq_T, *start_l, *end_l;
-    const i64 *ta_off, *tg_off, *gf_off, *gu_off, *pu_off, *tx_off;
-    const int2* m_pos;
+    const i64 *ta_off, *tg_off, *gf_off, *gu_off, *pu_off;
     const int *rowptr_f, *rowptr_b;
     const uint2 *fwd_rec, *bwd_rec;
-    const int4* q_rec;
+    const int4* m_rec;  // {from | to << 16, position in ascending edge index, class slot, weight}, ordered by class
     const int *m_ptr, *slot_emis, *order;
     i64 T, B, F;
     int r0, r1;  // rank range (a group of sequences) this launch works on
@@ -1303,10 +1292,7 @@ __global__ void __launch_bounds__(1024) k_sweep(RunArgs a, int smax, int dpmax, 
     if (RING > 0) cp_async_wait<0>();
 }
 
-constexpr int kPostBatch = 8;  // edges whose lines are loaded together
-// lines of edge scores a k_norm warp keeps in flight beyond the ones it is folding: the fold is a
-// chain of dependent steps fed from DRAM, and its only parallelism is how far ahead it loads
-constexpr int kNormBatch = 16;
+constexpr int kPostBatch = 4;  // edges whose lines are loaded together (the next ones' records with them)
 
 // decode a work unit (sequence, 32-frame tile) from its index in rank order
 struct PostUnit {
@@ -1329,173 +1315,232 @@ __device__ __forceinline__ PostUnit post_unit(const RunArgs& a, i64 u) {
     return p;
 }
 
-// Edge scores of every (frame, edge):
-//   x_e = ((alpha_t(from) + w) + score_t(emission)) + beta_{t+1}(to)              (fbw_op.cu:93-100)
-// written as X[tile][edge in ascending edge index][frame].  An unreachable source or target state
-// has score +inf and so has the sum, which is what the reference stores for such an edge
-// (fbw_op.cu:82-85).  One CTA per (sequence, 32-frame tile), lane = frame; in the tiled layouts
-// every load and store of a warp is one 128-byte line.  Fully parallel: no fold here.
-// (the work of `nwarps` warps on one unit; `warp` is this warp's number among them)
-__device__ __forceinline__ void score_unit(const RunArgs& a, const PostUnit& p, int lane, int warp, int nwarps) {
-    {
-        const bool valid = p.k * kTile + lane < p.Te;
-        // every lane loads (a tile is allocated for all 32 frames); frames past the sequence's
-        // length hold unspecified values and get +inf
-        const float* __restrict__ Ab = a.A + a.ta_off[p.b] + (i64)p.k * p.Sb * kTile + lane;
-        const float* __restrict__ Bb = a.Bt + a.ta_off[p.b] + (i64)p.k * p.Sb * kTile + lane;
-        const float* __restrict__ Gb = a.Gt + a.tg_off[p.b] + (i64)p.k * p.Db * kTile + lane;
-        float* __restrict__ Xb = a.X + a.tx_off[p.b] + (i64)p.k * p.Eb * kTile + lane;
-        const int4* __restrict__ q = a.q_rec + p.e0;
-        for (int i0 = warp * kPostBatch; i0 < p.Eb; i0 += nwarps * kPostBatch) {
-            int4  r[kPostBatch];
-            float al[kPostBatch], be[kPostBatch], g[kPostBatch];
-#pragma unroll
-            for (int j = 0; j < kPostBatch; j++) r[j] = __ldg(q + min(i0 + j, p.Eb - 1));
-#pragma unroll
-            for (int j = 0; j < kPostBatch; j++) {
-                al[j] = Ab[r[j].x * kTile];
-                be[j] = Bb[r[j].y * kTile];
-                g[j]  = Gb[r[j].z * kTile];
-            }
-#pragma unroll
-            for (int j = 0; j < kPostBatch; j++) {
-                const float v = ((al[j] + __int_as_float(r[j].w)) + g[j]) + be[j];
-                if (i0 + j < p.Eb) Xb[(i64)(i0 + j) * kTile] = valid ? v : CUDART_INF_F;
-            }
-        }
+// Sum of scaled terms (minimum, sum of exp(minimum - term)): adds s2 * exp(-m2) to s * exp(-m).  A term
+// that is +inf or NaN adds nothing.
+__device__ __forceinline__ void add_term(float& m, float& s, float m2, float s2) {
+    const float e = ex2_approx(fabsf(m - m2) * -1.44269504f);  // 0 while the sum is empty (m = +inf)
+    if (m2 < m) {
+        s = fmaf(s, e, s2);
+        m = m2;
+    } else if (m2 < CUDART_INF_F) {
+        s = fmaf(s2, e, s);
     }
 }
 
-__global__ void __launch_bounds__(256) k_score(RunArgs a) {
+// Frame normalisers and class posteriors of one (sequence, 32-frame tile) per CTA step, lane = frame.
+//   x_e  = ((alpha_t(from) + w) + score_t(emission)) + beta_{t+1}(to)             (fbw_op.cu:93-100)
+//   sum  = log-sum over all edges of x_e; sums[t,b] = 0 where no path exists        (fbw_op.cu:115-129)
+//   post = -log sum over the class's edges of exp(-(x_e - sum))                     (fbw_op.cu:131-153)
+// The edges come in class order (m_rec), an equal share of them per warp.  Every edge score is formed once,
+// in the reference's order of operations, and enters its class's running (minimum, scaled sum); finished
+// classes enter the frame's.  All values stay differences to a base near them until the normaliser is
+// known, so neither the class sums nor the normaliser are rounded to the grid of the scores (~1e4).
+// A class whose edges lie in the shares of several warps (a CTC blank has nearly half of all edges) is put
+// aside as partial sums, head (the share's first class) and tail (its last), and merged by the warp in
+// whose share it starts.  The class values go where the class's score was (Gt, not needed any more); once
+// the normaliser is known they are read back and leave transposed, every frame's row of P contiguous.
+//
+// Bound by the loads of state scores from L2 (two 128-byte lines per edge, one per class).  Before, the edge
+// scores of all frames went through memory (written once, read twice, with a serial fold over a sequence's
+// edges per frame between), in three kernels.
+//
+// Sequences of at most kFoldEdges edges take the frame's sum as the reference forms it, a left fold in
+// ascending edge index rounded to the grid of the scores at every step (fbw_op.cu:115-118), over the edges
+// within e^-kFoldReach of the best: a smaller term changes no sum of that grid.  Such a fold loses the small
+// terms one by one, and posteriors come out up to 2e-4 too large (magnitude 1e3) as the reference's do; for
+// these sizes the results stay those of the reference and the fold is short (one warp, ~30 ns an edge).  For
+// longer lists the fold would be the longest part of the pass, and the scaled sum, which has no such
+// error, takes its place.
+constexpr int   kPostWarps = 8;
+constexpr int   kFoldEdges = 128;
+constexpr float kFoldReach = 20.f;
+__global__ void __launch_bounds__(32 * kPostWarps, 3) k_post(RunArgs a) {
+    constexpr int W = kPostWarps;
+    __shared__ float stage[W][kTile][kTile + 1];
+    __shared__ float hm[W][kTile], hs[W][kTile], tm[W][kTile], ts[W][kTile], bw[W][kTile], fm[W][kTile], fs[W][kTile];
+    __shared__ int hslot[W], tslot[W], owned[W];
+    __shared__ unsigned short kept[W][kFoldEdges / W + 1];
+    __shared__ int nkept[W];
+    extern __shared__ float xs[];  // edge scores [position][frame] of a sequence of at most kFoldEdges edges
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const i64 u0 = a.pu_off[a.r0], nunits = a.pu_off[a.r1] - u0;
     for (i64 idx = blockIdx.x; idx < nunits; idx += gridDim.x) {
         const PostUnit p = post_unit(a, u0 + idx);
-        if (!in_chunks(tile_done_chunk(p.k, p.Te, a.chunk_steps), a)) continue;
-        score_unit(a, p, lane, warp, 8);
-    }
-}
-
-// Frame normalisers: sum = left fold of prob_add over the sequence's edges in ascending edge index
-// (fbw_op.cu:115-118), sums[t,b] = isinf(sum) ? 0 : sum (fbw_op.cu:120-129).  One warp per
-// (sequence, 32-frame tile), lane = frame, streaming the tile's edge scores in storage order; the
-// next lines are loaded while the current ones are folded.  The raw sum (+inf for a dead frame) goes
-// to N.
-// Every unit is its own warp so that all the serial folds of a call run side by side.
-// (one warp folds one unit; returns the raw sum of the lane's frame)
-__device__ __forceinline__ float norm_unit(const RunArgs& a, const PostUnit& p, int lane) {
-    {
+        if (!in_chunks(tile_done_chunk(p.k, p.Te, a.chunk_steps), a)) continue;  // uniform in the CTA
         const int  t     = p.k * kTile + lane;
         const bool valid = t < p.Te;
-        const float* __restrict__ Xb = a.X + a.tx_off[p.b] + (i64)p.k * p.Eb * kTile + lane;
-        float acc = CUDART_INF_F;
-        float nx[kNormBatch];
+        // every lane loads (a tile is allocated for all 32 frames); frames past the sequence's length hold
+        // unspecified values and count as +inf
+        const float* __restrict__ Ab = a.A + a.ta_off[p.b] + (i64)p.k * p.Sb * kTile + lane;
+        const float* __restrict__ Bb = a.Bt + a.ta_off[p.b] + (i64)p.k * p.Sb * kTile + lane;
+        float* Gb = a.Gt + a.tg_off[p.b] + (i64)p.k * p.Db * kTile + lane;
+        const int4* __restrict__ rec = a.m_rec + p.e0;
+        const bool fold = p.Eb <= kFoldEdges;
+
+        // ---- classes of this warp's share of the edges ----
+        const int i0 = (int)((i64)warp * p.Eb / W), i1 = (int)((i64)(warp + 1) * p.Eb / W);
+        float base = CUDART_INF_F;                   // what this warp's class values are relative to
+        float nm = CUDART_INF_F, ns = 0.f;           // the share's part of the frame's sum
+        float cm = CUDART_INF_F, cs = 0.f;           // the running class
+        int   cur = -1, cnt = 0, head = -1, tail = -1;
+        auto store_class = [&](int slot, float m, float s, bool single) {
+            if (base == CUDART_INF_F && m < CUDART_INF_F) base = m;
+            const float v = (m - base) - (single ? 0.f : logf(s));
+            Gb[slot * kTile] = m == CUDART_INF_F ? CUDART_INF_F : v;
+        };
+        auto finish_class = [&]() {
+            add_term(nm, ns, cm, cs);
+            if (head < 0) {
+                head = cur;
+                hm[warp][lane] = cm;
+                hs[warp][lane] = cs;
+            } else {
+                store_class(cur, cm, cs, cnt == 1);
+            }
+        };
+        int4 rn[kPostBatch];  // the next batch's records: their loads go on beside the scores' loads
 #pragma unroll
-        for (int j = 0; j < kNormBatch; j++) nx[j] = j < p.Eb ? Xb[(i64)j * kTile] : CUDART_INF_F;
-        for (int i0 = 0; i0 < p.Eb; i0 += kNormBatch) {
-            float x[kNormBatch];
+        for (int j = 0; j < kPostBatch; j++) rn[j] = i0 < i1 ? __ldg(rec + min(i0 + j, i1 - 1)) : make_int4(0, 0, 0, 0);
+        for (int i = i0; i < i1; i += kPostBatch) {
+            int4  r[kPostBatch];
+            float al[kPostBatch], be[kPostBatch], g[kPostBatch];
 #pragma unroll
-            for (int j = 0; j < kNormBatch; j++) x[j] = nx[j];
-#pragma unroll
-            for (int j = 0; j < kNormBatch; j++) {
-                const int i = i0 + kNormBatch + j;
-                nx[j] = i < p.Eb ? Xb[(i64)i * kTile] : CUDART_INF_F;
+            for (int j = 0; j < kPostBatch; j++) {
+                r[j]  = rn[j];
+                rn[j] = __ldg(rec + min(i + kPostBatch + j, i1 - 1));
             }
 #pragma unroll
-            for (int j = 0; j < kNormBatch; j++) acc = prob_add(acc, x[j]);
-        }
-        if (valid) a.sums[(i64)t * a.B + p.b] = isinf(acc) ? 0.f : acc;
-        a.N[p.u * kTile + lane] = acc;
-        return acc;
-    }
-}
-
-__global__ void __launch_bounds__(128) k_norm(RunArgs a) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const i64 u0 = a.pu_off[a.r0], nunits = a.pu_off[a.r1] - u0;
-    const i64 W = (i64)gridDim.x * 4;
-    for (i64 idx = (i64)blockIdx.x * 4 + warp; idx < nunits; idx += W) {
-        const PostUnit p = post_unit(a, u0 + idx);
-        if (!in_chunks(tile_done_chunk(p.k, p.Te, a.chunk_steps), a)) continue;
-        norm_unit(a, p, lane);
-    }
-}
-
-// Class posteriors: post[t][slot] = -log sum over the slot's edges of exp(-(x_e - sum))
-// (fbw_op.cu:131-153), as a running (minimum, scaled sum) pair.  The terms are normalised
-// (magnitude of a log-posterior), so a fast exponential is accurate to ~1e-7 in the posterior; the
-// reference accumulates the same terms with atomics in no fixed order.  A slot with one edge gets
-// x_e - sum exactly.  One CTA per (sequence, 32-frame tile); each warp takes blocks of 32 slots,
-// lane = frame, and writes them out transposed so that every frame's row of P is contiguous.
-// (the work of `nwarps` warps on one unit; `st` is this warp's 32 x 33 staging tile, `acc` the raw
-// sum of the lane's frame)
-__device__ __forceinline__ void class_unit(const RunArgs& a, const PostUnit& p, int lane, int warp, int nwarps,
-                                           float (*st)[kTile + 1], float acc) {
-    {
-        const bool rowdead = !(acc < CUDART_INF_F);  // no path through this frame
-        const float* __restrict__ Xb = a.X + a.tx_off[p.b] + (i64)p.k * p.Eb * kTile + lane;
-        const int2* __restrict__ m  = a.m_pos + p.e0;
-        const int* __restrict__ mp  = a.m_ptr + p.so;
-        float* __restrict__ Pb      = a.P + a.gf_off[p.b];
-        const int mbase = mp[0];
-        for (int d0 = warp * kTile; d0 < p.Db; d0 += nwarps * kTile) {
-            const int nd = min(kTile, p.Db - d0);
-            const int j0 = mp[d0] - mbase, j1 = mp[d0 + nd] - mbase;
-            int   cur = -1;
-            float mn = CUDART_INF_F, sme = 1.f;
-            for (int i = j0; i < j1; i += kPostBatch) {
-                int2  r[kPostBatch];
-                float x[kPostBatch];
+            for (int j = 0; j < kPostBatch; j++) {
+                al[j] = Ab[(r[j].x & 0xffff) * kTile];
+                be[j] = Bb[((unsigned)r[j].x >> 16) * kTile];
+                g[j]  = Gb[r[j].z * kTile];
+            }
 #pragma unroll
-                for (int j = 0; j < kPostBatch; j++) r[j] = __ldg(m + min(i + j, j1 - 1));
-#pragma unroll
-                for (int j = 0; j < kPostBatch; j++) x[j] = Xb[(i64)r[j].x * kTile];
-#pragma unroll
-                for (int j = 0; j < kPostBatch; j++) {
-                    if (i + j >= j1) continue;   // past the end of the block (uniform)
-                    const float y = x[j] - acc;  // +inf for dead edges; NaN only if the row is dead
-                    if (r[j].y != cur) {         // uniform: a new slot starts
-                        if (cur >= 0) {
-                            st[cur - d0][lane] =
-                                (mn == CUDART_INF_F || rowdead) ? CUDART_INF_F : mn - logf(sme);
-                        }
-                        cur = r[j].y;
-                        mn  = y;
-                        sme = 1.f;
-                    } else {
-                        // running (minimum, sum scaled to it) without branches: the frames of a warp
-                        // disagree on which term is the smaller, and both sides of a branch would run
-                        const float nm = fminf(mn, y);
-                        const float t1 = nm < CUDART_INF_F ? __expf(nm - mn) : 0.f;  // exp(-inf) = 0 while mn = +inf
-                        const float t2 = y < CUDART_INF_F ? __expf(nm - y) : 0.f;
-                        sme = sme * t1 + t2;
-                        mn  = nm;
-                    }
+            for (int j = 0; j < kPostBatch; j++) {
+                if (i + j >= i1) continue;  // uniform
+                const float v = ((al[j] + __int_as_float(r[j].w)) + g[j]) + be[j];
+                const float x = valid ? v : CUDART_INF_F;
+                if (fold) xs[r[j].y * kTile + lane] = x;
+                if (r[j].z != cur) {  // uniform: a new class starts
+                    if (cur >= 0) finish_class();
+                    cur = r[j].z;
+                    cnt = 1;
+                    cm  = x;
+                    cs  = 1.f;
+                } else {
+                    add_term(cm, cs, x, 1.f);
+                    cnt++;
                 }
             }
-            if (cur >= 0) {
-                st[cur - d0][lane] = (mn == CUDART_INF_F || rowdead) ? CUDART_INF_F : mn - logf(sme);
+        }
+        if (cur >= 0) {  // the share's last class may go on in the next warp's share
+            add_term(nm, ns, cm, cs);
+            if (head < 0) {
+                head = cur;
+                hm[warp][lane] = cm;
+                hs[warp][lane] = cs;
+            } else {
+                tail = cur;
+                tm[warp][lane] = cm;
+                ts[warp][lane] = cs;
+            }
+        }
+        fm[warp][lane] = nm;
+        fs[warp][lane] = ns;
+        if (lane == 0) {
+            hslot[warp] = head;
+            tslot[warp] = tail;
+        }
+        __syncthreads();
+
+        // ---- the normaliser, and the classes that several warps share ----
+        nm = CUDART_INF_F;
+        ns = 0.f;
+#pragma unroll
+        for (int w = 0; w < W; w++) add_term(nm, ns, fm[w][lane], fs[w][lane]);
+        float logn = logf(ns);
+        if (fold) {
+            // the edges (ascending) that can move the sum of some frame of the tile: within kFoldReach of its
+            // smallest score
+            int n = 0;
+            for (int i = i0; i < i1; i++) {
+                if (__any_sync(0xffffffffu, xs[i * kTile + lane] <= fminf(nm + kFoldReach, 3.4e38f))) {
+                    if (lane == 0) kept[warp][n] = (unsigned short)i;
+                    n++;
+                }
+            }
+            if (lane == 0) nkept[warp] = n;
+            __syncthreads();
+            if (warp == 0) {
+                float acc = CUDART_INF_F;
+                for (int w = 0; w < W; w++) {
+                    const int nw = nkept[w];
+#pragma unroll 4
+                    for (int i = 0; i < nw; i++) acc = prob_add(acc, xs[kept[w][i] * kTile + lane]);
+                }
+                fm[0][lane] = acc;
+            }
+            __syncthreads();
+            nm = fm[0][lane];
+            logn = 0.f;
+        }
+        const bool  dead = !(nm < CUDART_INF_F);  // no path through this frame
+        if (warp == 0 && valid) a.sums[(i64)t * a.B + p.b] = dead ? 0.f : nm - logn;
+        int own = 0x7fffffff;  // first class whose value this warp writes
+        if (head >= 0) {
+            int before = -1;  // the class that is running when this warp's share begins
+            for (int w = warp - 1; w >= 0; w--) {
+                if (hslot[w] >= 0) {
+                    before = tslot[w] >= 0 ? tslot[w] : hslot[w];
+                    break;
+                }
+            }
+            auto with_heads = [&](int slot, float m, float s) {  // ... of the following shares
+                for (int w = warp + 1; w < W; w++) {
+                    if (hslot[w] < 0) continue;  // an empty share
+                    if (hslot[w] != slot) break;
+                    add_term(m, s, hm[w][lane], hs[w][lane]);
+                    if (tslot[w] >= 0) break;  // the class ends in that share
+                }
+                store_class(slot, m, s, false);
+            };
+            const bool starts = before != head;
+            if (starts && tail >= 0) store_class(head, hm[warp][lane], hs[warp][lane], false);
+            if (starts && tail < 0) with_heads(head, hm[warp][lane], hs[warp][lane]);
+            if (tail >= 0) with_heads(tail, tm[warp][lane], ts[warp][lane]);
+            if (starts) own = head;
+            else if (tail >= 0) own = head + 1;
+        }
+        bw[warp][lane] = base;
+        if (lane == 0) owned[warp] = own;
+        __syncthreads();
+
+        // ---- posteriors, transposed: frame r of the tile gets its classes as one contiguous write ----
+        float* __restrict__ Pb = a.P + a.gf_off[p.b];
+        float (*st)[kTile + 1] = stage[warp];
+        for (int d0 = warp * kTile; d0 < p.Db; d0 += W * kTile) {
+            const int nd = min(kTile, p.Db - d0);
+            int w = 0;
+            for (int q = 1; q < W; q++) w = owned[q] <= d0 ? q : w;
+            float shift = bw[w][lane] - nm;
+#pragma unroll 8
+            for (int d = 0; d < nd; d++) {
+                const float x = Gb[(d0 + d) * kTile];
+                bool moved = false;
+                for (int q = w + 1; q < W; q++) {
+                    if (owned[q] == d0 + d) { w = q; moved = true; }
+                }
+                if (moved) shift = bw[w][lane] - nm;
+                st[d][lane] = dead || x == CUDART_INF_F ? CUDART_INF_F : (x + shift) + logn;
             }
             __syncwarp();
-            // transpose: frame r of the tile gets its nd posteriors as one contiguous write
             for (int r = 0; r < kTile; r++) {
                 const int tr = p.k * kTile + r;
                 if (tr < p.Te && lane < nd) Pb[(i64)tr * p.Dp + d0 + lane] = st[lane][r];
             }
             __syncwarp();
         }
-    }
-}
-
-constexpr int kClassWarps = 8;  // warps of a k_class CTA: blocks of 32 slots of one unit in flight
-__global__ void __launch_bounds__(32 * kClassWarps) k_class(RunArgs a) {
-    __shared__ float stage[kClassWarps][kTile][kTile + 1];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const i64 u0 = a.pu_off[a.r0], nunits = a.pu_off[a.r1] - u0;
-    for (i64 idx = blockIdx.x; idx < nunits; idx += gridDim.x) {
-        const PostUnit p = post_unit(a, u0 + idx);
-        if (!in_chunks(tile_done_chunk(p.k, p.Te, a.chunk_steps), a)) continue;
-        class_unit(a, p, lane, warp, kClassWarps, stage[warp], a.N[p.u * kTile + lane]);
+        __syncthreads();
     }
 }
 
@@ -1735,7 +1780,7 @@ __global__ void __launch_bounds__(1024) k_loss(const float* __restrict__ sums, i
 // host side
 // ---------------------------------------------------------------------------------------------
 struct RunLayout {
-    size_t A, Bt, Gt, Gf, Gs, P, X, N, carry, next_row, total;
+    size_t A, Bt, Gt, Gf, Gs, P, carry, next_row, total;
 };
 
 RunLayout run_layout(const fbw_b200_summary& s) {
@@ -1752,8 +1797,6 @@ RunLayout run_layout(const fbw_b200_summary& s) {
     L.Gf    = take((size_t)s.frame_floats);
     L.Gs    = take((size_t)s.frame_floats * 2);
     L.P     = take((size_t)s.frame_floats);
-    L.X     = take((size_t)s.score_floats);
-    L.N     = take((size_t)s.post_units * kTile);
     L.carry = take((size_t)(4 * s.S));
     L.next_row = take(2 * FBW_B200_GROUPS);  // a 64-bit row counter per group (background_rows)
     L.total = off;
@@ -1799,13 +1842,11 @@ void plan_args(RunArgs& a, const void* plan, const fbw_b200_summary& s) {
     a.gf_off = at<i64>(plan, L.gf_off);
     a.gu_off = at<i64>(plan, L.gu_off);
     a.pu_off = at<i64>(plan, L.pu_off);
-    a.tx_off = at<i64>(plan, L.tx_off);
-    a.m_pos  = at<int2>(plan, L.m_pos);
     a.rowptr_f = at<int>(plan, L.rowptr_f);
     a.rowptr_b = at<int>(plan, L.rowptr_b);
     a.fwd_rec  = at<uint2>(plan, L.fwd_rec);
     a.bwd_rec  = at<uint2>(plan, L.bwd_rec);
-    a.q_rec    = at<int4>(plan, L.q_rec);
+    a.m_rec    = at<int4>(plan, L.m_rec);
     a.m_ptr     = at<int>(plan, L.m_ptr);
     a.slot_emis = at<int>(plan, L.slot_emis);
     a.order     = at<int>(plan, L.order);
@@ -1832,8 +1873,6 @@ RunArgs fbw_args(const void* plan, const fbw_b200_summary& s, void* work, const 
     a.Gf = at<float>(work, R.Gf);
     a.Gs = at<float2>(work, R.Gs);
     a.P  = at<float>(work, R.P);
-    a.X  = at<float>(work, R.X);
-    a.N  = at<float>(work, R.N);
     a.carry = at<float>(work, R.carry);
     a.fused = fused;
     return a;
@@ -1874,8 +1913,8 @@ int sm_count() {
 // Raise a kernel's dynamic shared-memory limit to `smem` bytes unless an earlier launch on this
 // device already raised it that far (`granted` is the per-device record of one kernel).
 template <typename Kernel>
-cudaError_t grant_smem(Kernel kernel, std::atomic<int>* granted, size_t smem) {
-    if (smem <= 48 * 1024) return cudaSuccess;
+cudaError_t grant_smem(Kernel kernel, std::atomic<int>* granted, size_t smem, size_t fixed = 0) {
+    if (smem + fixed <= 48 * 1024) return cudaSuccess;  // (fixed: the kernel's static shared memory)
     const int dev = current_device();
     if ((size_t)granted[dev].load(std::memory_order_relaxed) >= smem) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -2194,14 +2233,12 @@ int launch_group(RunArgs a, int r0, int r1, i64 ms, i64 me, i64 md, const fbw_b2
     if (ev) CUDA_OK(cudaEventRecord(ev[2], st));
     if ((what & kDoPost) && s.post_units > 0) {
         const i64 units = tiles * nb;  // upper bound; the kernels read the exact count
-        int g1 = (int)(units < (i64)sms * 8 ? units : (i64)sms * 8);
-        i64 w2 = (units + 3) / 4;
-        int g2 = (int)(w2 < (i64)sms * 16 ? w2 : (i64)sms * 16);
-        int g3 = (int)(units < (i64)sms * 6 ? units : (i64)sms * 6);
-        k_score<<<g1 > 0 ? g1 : 1, 256, 0, st>>>(a);
-        k_norm<<<g2 > 0 ? g2 : 1, 128, 0, st>>>(a);
-        k_class<<<g3 > 0 ? g3 : 1, 32 * kClassWarps, 0, st>>>(a);
-        COUNT_LAUNCH(3);
+        const int grid = (int)(units < (i64)sms * 6 ? units : (i64)sms * 6);
+        const size_t xs = sizeof(float) * kTile * (size_t)(me < kFoldEdges ? me : kFoldEdges);
+        static std::atomic<int> granted[kMaxDevices];
+        CUDA_OK(grant_smem(k_post, granted, sizeof(float) * kTile * kFoldEdges, 42 * 1024));
+        k_post<<<grid > 0 ? grid : 1, 32 * kPostWarps, xs, st>>>(a);
+        COUNT_LAUNCH(1);
     }
     if (ev) CUDA_OK(cudaEventRecord(ev[3], st));
     if (what & kDoPatch) {
@@ -2330,8 +2367,7 @@ static int prepare_impl(const int32_t* edges, const float* weights, const int32_
             edges, weights, E, F, at<int>(plan, L.qe), at<int>(plan, L.edge_off),
             at<int>(plan, L.state_off), at<int>(plan, L.packed_of), at<int>(plan, L.rowptr_f),
             at<int>(plan, L.rowptr_b), at<uint2>(plan, L.fwd_rec), at<uint2>(plan, L.bwd_rec),
-            at<int4>(plan, L.q_rec), at<int2>(plan, L.m_pos),
-            at<int>(plan, L.m_ptr), at<int>(plan, L.slot_emis), at<int>(plan, L.slot_off),
+            at<int4>(plan, L.m_rec), at<int>(plan, L.m_ptr), at<int>(plan, L.slot_emis), at<int>(plan, L.slot_off),
             at<int>(plan, L.nslot), hdr);
     } else if (E > 0) {
         k_edgekeys<<<blocks(E), TB, 0, st>>>(edges, E, F, at<int>(plan, L.packed_of),
@@ -2388,10 +2424,10 @@ static int prepare_impl(const int32_t* edges, const float* weights, const int32_
     if (E > 0 && !fast) {
         k_records<<<blocks(E), TB, 0, st>>>(
             edges, weights, E, at<int>(plan, L.packed_of), at<int>(plan, L.state_off),
-            at<int>(plan, L.slot_off), at<int>(plan, L.slot_of_edge), at<int>(plan, L.qe),
+            at<int>(plan, L.slot_off), at<int>(plan, L.slot_of_edge),
             at<int>(plan, L.fe), at<int>(plan, L.be), at<int>(plan, L.me), at<int>(plan, L.qpos),
             at<int>(plan, L.edge_off), at<uint2>(plan, L.fwd_rec), at<uint2>(plan, L.bwd_rec),
-            at<int4>(plan, L.q_rec), at<int2>(plan, L.m_pos), hdr);
+            at<int4>(plan, L.m_rec), hdr);
     }
     CUDA_OK(cudaGetLastError());
     return FBW_B200_OK;
