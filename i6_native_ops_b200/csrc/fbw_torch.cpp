@@ -234,9 +234,21 @@ std::vector<torch::Tensor> fbw_host_scores(torch::Tensor& am_scores, torch::Tens
     return {out, sums, loss2};
 }
 
+static std::vector<torch::Tensor> run_fused_impl(const Prepared& p, const torch::Tensor& log_probs,
+                                                 const torch::Tensor& grad, const torch::Tensor& sums) {
+    auto stream = at::cuda::getCurrentCUDAStream();
+    size_t wbytes = fbw_b200_run_bytes(&p.summary);
+    torch::Tensor work = byte_buffer(wbytes, log_probs.device());
+    check_status(fbw_b200_run_fused(p.plan.data_ptr(), &p.summary, log_probs.data_ptr<float>(),
+                                    grad.data_ptr<float>(), sums.data_ptr<float>(), nullptr,
+                                    work.data_ptr(), wbytes,
+                                    reinterpret_cast<fbw_b200_stream_t>(stream.stream())));
+    return {grad, sums};
+}
+
 // The op with the wrapper's passes folded in: log_probs (B,T,F) as the caller holds them ->
 // [grad (B,T,F) = -posterior, sum_output (T,B)].  Replaces neg/transpose/contiguous before the op
-// and neg/exp after it (i6_native_ops/fbw/__init__.py:41-44, 66); opt-in, used by fbw_loss_fused.
+// and neg/exp after it (i6_native_ops/fbw/__init__.py:41-44, 66); used by fbw_loss.
 std::vector<torch::Tensor> fbw_fused(torch::Tensor& log_probs, torch::Tensor& edges,
                                      torch::Tensor& weights, torch::Tensor& start_end_states,
                                      torch::Tensor& seq_lens, int64_t num_states) {
@@ -248,17 +260,11 @@ std::vector<torch::Tensor> fbw_fused(torch::Tensor& log_probs, torch::Tensor& ed
     check_same_device(log_probs, edges);
     c10::cuda::CUDAGuard guard(log_probs.device());
     const int64_t B = log_probs.size(0), T = log_probs.size(1), F = log_probs.size(2);
+    // the outputs do not depend on the plan: allocate them while the plan is still being built
     torch::Tensor grad = torch::empty_like(log_probs);
     torch::Tensor sums = torch::empty({T, B}, log_probs.options());
     Prepared p = prepare_impl(edges, weights, start_end_states, seq_lens, T, F, num_states);
-    auto stream = at::cuda::getCurrentCUDAStream();
-    size_t wbytes = fbw_b200_run_bytes(&p.summary);
-    torch::Tensor work = byte_buffer(wbytes, log_probs.device());
-    check_status(fbw_b200_run_fused(p.plan.data_ptr(), &p.summary, log_probs.data_ptr<float>(),
-                                    grad.data_ptr<float>(), sums.data_ptr<float>(), nullptr,
-                                    work.data_ptr(), wbytes,
-                                    reinterpret_cast<fbw_b200_stream_t>(stream.stream())));
-    return {grad, sums};
+    return run_fused_impl(p, log_probs, grad, sums);
 }
 
 // Two-step form of the same op for callers that reuse one batch of automata with new scores:
@@ -300,6 +306,18 @@ std::vector<torch::Tensor> fbw_run(const PlanHandle& h, torch::Tensor& am_scores
     TORCH_CHECK(am_scores.device() == h.p.plan.device(), "am_scores and plan on different devices");
     c10::cuda::CUDAGuard guard(am_scores.device());
     return run_impl(h.p, am_scores, true);
+}
+
+// fbw_run with the wrapper's passes folded in (see fbw_fused): log_probs (B,T,F) -> [grad, sum_output]
+std::vector<torch::Tensor> fbw_run_fused(const PlanHandle& h, torch::Tensor& log_probs) {
+    check_input(log_probs, torch::kFloat32, "log_probs");
+    const fbw_b200_summary& s = h.p.summary;
+    TORCH_CHECK(log_probs.dim() == 3 && log_probs.size(0) == s.B && log_probs.size(1) == s.T &&
+                    log_probs.size(2) == s.F,
+                "log_probs must have the (B, T, F) the plan was prepared for");
+    TORCH_CHECK(log_probs.device() == h.p.plan.device(), "log_probs and plan on different devices");
+    c10::cuda::CUDAGuard guard(log_probs.device());
+    return run_fused_impl(h.p, log_probs, torch::empty_like(log_probs), torch::empty({s.T, s.B}, log_probs.options()));
 }
 
 // fbw_run with per-kernel device times: returns ([out, sum_output, loss2], [ms per phase]).
@@ -402,6 +420,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           py::arg("seq_lens"), py::arg("num_states"), py::arg("out") = py::none(), py::arg("staged") = true);
     m.def("fbw_prepare", &fbw_prepare, "Validate and sort a batch of automata");
     m.def("fbw_run", &fbw_run, "Run fbw on prepared automata");
+    m.def("fbw_run_fused", &fbw_run_fused, "fbw_fused on prepared automata");
     m.def("abi_version", []() { return fbw_b200_abi_version(); });
 
     py::class_<DebugOptions>(m, "DebugOptions", py::module_local())
