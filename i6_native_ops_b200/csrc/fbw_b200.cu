@@ -497,6 +497,25 @@ __global__ void k_slots(const unsigned long long* __restrict__ key64s, const int
     }
 }
 
+// exclusive sums of a row of n values in shared memory to dst (may be null) by one warp; returns the total
+__device__ __forceinline__ i64 warp_offsets(const i64* row, int n, i64* dst) {
+    const int lane = threadIdx.x & 31;
+    i64 carry = 0;
+    for (int base = 0; base < n; base += 32) {
+        const int b = base + lane;
+        const i64 v = b < n ? row[b] : 0;
+        i64 sum = v;
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) {
+            const i64 o = __shfl_up_sync(0xffffffffu, sum, k);
+            if (lane >= k) sum += o;
+        }
+        if (b < n && dst) dst[b] = carry + sum - v;
+        carry += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    return carry;
+}
+
 // single block: everything per sequence that needs the slot counts.  Storage offsets of the run
 // arrays are scans in sequence order; work-item offsets (gather and posterior units) are scans in
 // RANK order, rank 0 being the most expensive sequence (frames x edges), so that kernels hand out
@@ -518,6 +537,12 @@ __global__ void __launch_bounds__(1024) k_off2(const int* __restrict__ state_off
     __shared__ int smax[4];
     __shared__ int smin;
     __shared__ int gmax[3][FBW_B200_GROUPS];
+    // The eight offset arrays of up to kRowSeqs sequences are scanned by a warp each, side by side (64
+    // sequences: see k_off2's duration in the table of kernels); larger batches by the block, one by one.
+    constexpr int kRowSeqs = 512;
+    __shared__ i64 rows[6][kRowSeqs];
+    const bool in_rows = B <= kRowSeqs;
+    const int  warp = threadIdx.x >> 5;
     if (threadIdx.x < 8) carry[threadIdx.x] = 0;
     if (threadIdx.x < 4) smax[threadIdx.x] = 0;
     if (threadIdx.x == 0) smin = 0x7fffffff;
@@ -559,6 +584,18 @@ __global__ void __launch_bounds__(1024) k_off2(const int* __restrict__ state_off
             if (Te > 0) atomicMin(&smin, Te);
         }
         i64* dst[6] = {ta_off, tg_off, gf_off, nullptr, tx_off, nullptr};
+        if (in_rows) {
+            if (ok) {
+                for (int k = 0; k < 6; k++) rows[k][b] = v[k];
+            }
+            __syncthreads();
+            if (warp < 6) {
+                i64* to = warp == 0 ? ta_off : (warp == 1 ? tg_off : (warp == 2 ? gf_off : (warp == 4 ? tx_off : nullptr)));
+                const i64 total = warp_offsets(rows[warp], B, to);
+                if ((threadIdx.x & 31) == 0) carry[warp] = total;
+            }
+            break;
+        }
         for (int k = 0; k < 6; k++) {
             i64 ex, agg;
             Scan(tmp).ExclusiveSum(v[k], ex, agg);
@@ -574,6 +611,7 @@ __global__ void __launch_bounds__(1024) k_off2(const int* __restrict__ state_off
     for (int b = threadIdx.x; b < B; b += 1024) {
         const i64 cb = cost[b];
         int rank = 0;
+#pragma unroll 8
         for (int j = 0; j < B; j++) {
             const i64 cj = cost[j];
             rank += (cj > cb || (cj == cb && j < b)) ? 1 : 0;
@@ -601,6 +639,19 @@ __global__ void __launch_bounds__(1024) k_off2(const int* __restrict__ state_off
             atomicMax(&gmax[2][g], Db);
         }
         i64* dst[2] = {gu_off, pu_off};
+        if (in_rows) {
+            if (ok) {
+                rows[0][r] = v[0];
+                rows[1][r] = v[1];
+            }
+            __syncthreads();
+            if (warp < 2) {
+                const i64 total = warp_offsets(rows[warp], B, warp == 0 ? gu_off : pu_off);
+                if ((threadIdx.x & 31) == 0) carry[6 + warp] = total;
+            }
+            __syncthreads();
+            break;
+        }
         for (int k = 0; k < 2; k++) {
             i64 ex, agg;
             Scan(tmp).ExclusiveSum(v[k], ex, agg);
@@ -658,11 +709,17 @@ __global__ void k_seqkeys(const int* __restrict__ edges, i64 E, unsigned* keyq, 
     }
 }
 
-typedef cub::BlockRadixSort<unsigned, kFastThreads, kFastItems> FastSort;
-typedef cub::BlockScan<int, kFastThreads>                       FastScan;
+// A sequence's edges are sorted with kFastItems per thread, or with kFewItems where that is enough.  Keys
+// are (state or emission, position) and come in the order of their positions; the radix sort is stable, so
+// only the upper part is sorted, and of that only the bits that occur.
+constexpr int kFewItems = 2;
+template <int ITEMS>
+using FastSort = cub::BlockRadixSort<unsigned, kFastThreads, ITEMS>;
+typedef cub::BlockScan<int, kFastThreads> FastScan;
 struct FastSmem {
     union {
-        typename FastSort::TempStorage sort;
+        typename FastSort<kFastItems>::TempStorage sort;
+        typename FastSort<kFewItems>::TempStorage  sort_few;
         typename FastScan::TempStorage scan;
     } t;
     unsigned sorted[kFastCap];     // the keys of the last sort, in order
@@ -671,6 +728,121 @@ struct FastSmem {
     unsigned last[kFastThreads];   // each thread's last sorted key (for the head test)
     int      deg_max;
 };
+
+// the three sorted lists of a sequence (see k_seqsort)
+template <int ITEMS>
+__device__ __forceinline__ void seqsort_lists(
+    FastSmem& sm, const float* weights, i64 F, const int* qe, int e0, int Eb, int s0, int Sb, int so, int b,
+    int* rowptr_f, int* rowptr_b, uint2* fwd_rec, uint2* bwd_rec, int4* m_rec, int* m_ptr, int* slot_emis,
+    int* nslot, fbw_b200_summary* hdr) {
+    const int tid = threadIdx.x;
+    // (past-the-end keys are all ones: not below any key in the sorted bits, and behind their equals)
+    auto sort = [&](unsigned (&k)[ITEMS], int bits) {
+        if constexpr (ITEMS == kFewItems) {
+            FastSort<ITEMS>(sm.t.sort_few).Sort(k, kFastPosBits, kFastPosBits + bits);
+        } else {
+            FastSort<ITEMS>(sm.t.sort).Sort(k, kFastPosBits, kFastPosBits + bits);
+        }
+    };
+    auto bits_of = [](i64 n) { return min(32 - kFastPosBits, 32 - __clz((int)max(n - 1, (i64)1))); };
+    const unsigned pos_mask = (1u << kFastPosBits) - 1u;
+    unsigned keys[ITEMS];
+
+    // ---- slots: sort by (emission, position) ----
+#pragma unroll
+    for (int k = 0; k < ITEMS; k++) {
+        const int i = tid * ITEMS + k;
+        keys[k] = i < Eb ? ((unsigned)sm.emis[i] << kFastPosBits) | (unsigned)i : 0xffffffffu;
+    }
+    sort(keys, bits_of(F));
+    sm.last[tid] = keys[ITEMS - 1];
+    __syncthreads();
+    int heads = 0;
+    bool head[ITEMS];
+#pragma unroll
+    for (int k = 0; k < ITEMS; k++) {
+        const int j = tid * ITEMS + k;
+        const unsigned prev = k > 0 ? keys[k - 1] : (tid > 0 ? sm.last[tid - 1] : 0xffffffffu);
+        head[k] = j < Eb && (j == 0 || (keys[k] >> kFastPosBits) != (prev >> kFastPosBits));
+        heads += head[k] ? 1 : 0;
+    }
+    int before, total;
+    FastScan(sm.t.scan).ExclusiveSum(heads, before, total);
+    {
+        int slot = before - 1;
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            const int j = tid * ITEMS + k;
+            if (j >= Eb) break;
+            if (head[k]) {
+                slot++;
+                slot_emis[so + slot] = (int)(keys[k] >> kFastPosBits);
+                m_ptr[so + slot]     = e0 + j;
+            }
+            const int i = (int)(keys[k] & pos_mask);
+            sm.slot[i] = (unsigned short)slot;
+            m_rec[e0 + j] = make_int4((int)(sm.from[i] | ((unsigned)sm.to[i] << 16)), i, slot, __float_as_int(weights[qe[e0 + i]]));
+        }
+    }
+    if (tid == 0) {
+        m_ptr[so + total] = e0 + Eb;
+        nslot[b]          = total;
+    }
+    __syncthreads();
+
+    // ---- forward list (by target state) and backward list (by source state) ----
+    for (int dir = 0; dir < 2; dir++) {
+        const unsigned short* key_state = dir == 0 ? sm.to : sm.from;
+        const unsigned short* other     = dir == 0 ? sm.from : sm.to;
+        int*   rowptr = dir == 0 ? rowptr_f : rowptr_b;
+        uint2* rec    = dir == 0 ? fwd_rec : bwd_rec;
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            const int i = tid * ITEMS + k;
+            keys[k] = i < Eb ? ((unsigned)key_state[i] << kFastPosBits) | (unsigned)i : 0xffffffffu;
+        }
+        __syncthreads();  // the previous use of the sort storage is over
+        sort(keys, bits_of(Sb));
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            const int j = tid * ITEMS + k;
+            sm.sorted[j] = keys[k];
+            if (j < Eb) {
+                const int i = (int)(keys[k] & pos_mask);
+                rec[e0 + j] = make_uint2((unsigned)other[i] | ((unsigned)sm.slot[i] << 16),
+                                         __float_as_uint(weights[qe[e0 + i]]));
+            }
+        }
+        __syncthreads();
+        // row pointers: first position whose state is >= s; the entry after the last state is the
+        // first entry of the next sequence (both write the same value)
+        int dmax = 0;
+        for (int s = tid; s <= Sb; s += kFastThreads) {
+            const unsigned want = (unsigned)s << kFastPosBits;
+            int lo = 0, hi = Eb;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (sm.sorted[mid] < want) lo = mid + 1; else hi = mid;
+            }
+            rowptr[s0 + s] = e0 + lo;
+            if (s < Sb) {
+                const unsigned nxt = (unsigned)(s + 1) << kFastPosBits;
+                int l2 = lo, h2 = Eb;
+                while (l2 < h2) {
+                    const int mid = (l2 + h2) >> 1;
+                    if (sm.sorted[mid] < nxt) l2 = mid + 1; else h2 = mid;
+                }
+                dmax = max(dmax, l2 - lo);
+            }
+        }
+        if (dmax > 0) atomicMax(&sm.deg_max, dmax);
+        __syncthreads();
+    }
+    if (tid == 0 && sm.deg_max > 0) {
+        atomicMax((unsigned long long*)&hdr->max_degree, (unsigned long long)sm.deg_max);
+    }
+}
+
 
 // Builds everything the run kernels need for sequence b = blockIdx.x from the sequence-grouped edge
 // list qe (ascending edge index inside the sequence): local slot numbers (distinct emissions in
@@ -706,101 +878,12 @@ __global__ void __launch_bounds__(kFastThreads) k_seqsort(
         sm.emis[i] = edges[2 * E + e];
     }
     __syncthreads();
-    const unsigned pos_mask = (1u << kFastPosBits) - 1u;
-    unsigned keys[kFastItems];
-
-    // ---- slots: sort by (emission, position) ----
-#pragma unroll
-    for (int k = 0; k < kFastItems; k++) {
-        const int i = tid * kFastItems + k;
-        keys[k] = i < Eb ? ((unsigned)sm.emis[i] << kFastPosBits) | (unsigned)i : 0xffffffffu;
-    }
-    FastSort(sm.t.sort).Sort(keys);
-    sm.last[tid] = keys[kFastItems - 1];
-    __syncthreads();
-    int heads = 0;
-    bool head[kFastItems];
-#pragma unroll
-    for (int k = 0; k < kFastItems; k++) {
-        const int j = tid * kFastItems + k;
-        const unsigned prev = k > 0 ? keys[k - 1] : (tid > 0 ? sm.last[tid - 1] : 0xffffffffu);
-        head[k] = j < Eb && (j == 0 || (keys[k] >> kFastPosBits) != (prev >> kFastPosBits));
-        heads += head[k] ? 1 : 0;
-    }
-    int before, total;
-    FastScan(sm.t.scan).ExclusiveSum(heads, before, total);
-    {
-        int slot = before - 1;
-#pragma unroll
-        for (int k = 0; k < kFastItems; k++) {
-            const int j = tid * kFastItems + k;
-            if (j >= Eb) break;
-            if (head[k]) {
-                slot++;
-                slot_emis[so + slot] = (int)(keys[k] >> kFastPosBits);
-                m_ptr[so + slot]     = e0 + j;
-            }
-            const int i = (int)(keys[k] & pos_mask);
-            sm.slot[i] = (unsigned short)slot;
-            m_rec[e0 + j] = make_int4((int)(sm.from[i] | ((unsigned)sm.to[i] << 16)), i, slot, __float_as_int(weights[qe[e0 + i]]));
-        }
-    }
-    if (tid == 0) {
-        m_ptr[so + total] = e0 + Eb;
-        nslot[b]          = total;
-    }
-    __syncthreads();
-
-    // ---- forward list (by target state) and backward list (by source state) ----
-    for (int dir = 0; dir < 2; dir++) {
-        const unsigned short* key_state = dir == 0 ? sm.to : sm.from;
-        const unsigned short* other     = dir == 0 ? sm.from : sm.to;
-        int*   rowptr = dir == 0 ? rowptr_f : rowptr_b;
-        uint2* rec    = dir == 0 ? fwd_rec : bwd_rec;
-#pragma unroll
-        for (int k = 0; k < kFastItems; k++) {
-            const int i = tid * kFastItems + k;
-            keys[k] = i < Eb ? ((unsigned)key_state[i] << kFastPosBits) | (unsigned)i : 0xffffffffu;
-        }
-        __syncthreads();  // the previous use of the sort storage is over
-        FastSort(sm.t.sort).Sort(keys);
-#pragma unroll
-        for (int k = 0; k < kFastItems; k++) {
-            const int j = tid * kFastItems + k;
-            sm.sorted[j] = keys[k];
-            if (j < Eb) {
-                const int i = (int)(keys[k] & pos_mask);
-                rec[e0 + j] = make_uint2((unsigned)other[i] | ((unsigned)sm.slot[i] << 16),
-                                         __float_as_uint(weights[qe[e0 + i]]));
-            }
-        }
-        __syncthreads();
-        // row pointers: first position whose state is >= s; the entry after the last state is the
-        // first entry of the next sequence (both write the same value)
-        int dmax = 0;
-        for (int s = tid; s <= Sb; s += kFastThreads) {
-            const unsigned want = (unsigned)s << kFastPosBits;
-            int lo = 0, hi = Eb;
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (sm.sorted[mid] < want) lo = mid + 1; else hi = mid;
-            }
-            rowptr[s0 + s] = e0 + lo;
-            if (s < Sb) {
-                const unsigned nxt = (unsigned)(s + 1) << kFastPosBits;
-                int l2 = lo, h2 = Eb;
-                while (l2 < h2) {
-                    const int mid = (l2 + h2) >> 1;
-                    if (sm.sorted[mid] < nxt) l2 = mid + 1; else h2 = mid;
-                }
-                dmax = max(dmax, l2 - lo);
-            }
-        }
-        if (dmax > 0) atomicMax(&sm.deg_max, dmax);
-        __syncthreads();
-    }
-    if (tid == 0 && sm.deg_max > 0) {
-        atomicMax((unsigned long long*)&hdr->max_degree, (unsigned long long)sm.deg_max);
+    if (Eb <= kFastThreads * kFewItems) {
+        seqsort_lists<kFewItems>(sm, weights, F, qe, e0, Eb, s0, Sb, so, b, rowptr_f, rowptr_b, fwd_rec, bwd_rec,
+                                 m_rec, m_ptr, slot_emis, nslot, hdr);
+    } else {
+        seqsort_lists<kFastItems>(sm, weights, F, qe, e0, Eb, s0, Sb, so, b, rowptr_f, rowptr_b, fwd_rec, bwd_rec,
+                                  m_rec, m_ptr, slot_emis, nslot, hdr);
     }
 }
 
