@@ -68,7 +68,6 @@ struct PlanLayout {
     size_t seq_T, start_l, end_l, nslot;                                         // int[B]
     size_t ta_off, tg_off, gf_off, gu_off, pu_off;                               // i64[B+1]
     size_t order, cost;                                                          // int[B], i64[B]
-    size_t tx_off;                                                               // i64[B+1]
     size_t qpos;                                                                 // int[E]
     size_t eiota, keyq, keyf, keyb, key32_out, qe, fe, be, me, slot_of_edge;     // [E]
     size_t key64, key64_out;                                                     // u64[E]
@@ -137,7 +136,6 @@ PlanLayout plan_layout(i64 B, i64 E, i64 S) {
     L.pu_off       = take(8 * (nB + 1));
     L.order        = take(4 * nB);
     L.cost         = take(8 * nB);
-    L.tx_off       = take(8 * (nB + 1));
     L.qpos         = take(4 * nE);
     L.eiota        = take(4 * nE);
     L.keyq         = take(4 * nE);
@@ -529,7 +527,7 @@ __global__ void __launch_bounds__(1024) k_off2(const int* __restrict__ state_off
                                               i64 F, i64 E, i64 S, int* slot_off, int* nslot,
                                               int* start_l,
                                               int* end_l, i64* ta_off, i64* tg_off, i64* gf_off,
-                                              i64* gu_off, i64* pu_off, i64* tx_off, i64* cost,
+                                              i64* gu_off, i64* pu_off, i64* cost,
                                               int* order, int fast, fbw_b200_summary* hdr) {
     typedef cub::BlockScan<i64, 1024> Scan;
     __shared__ typename Scan::TempStorage tmp;
@@ -583,14 +581,14 @@ __global__ void __launch_bounds__(1024) k_off2(const int* __restrict__ state_off
             atomicMax(&smax[3], Te);
             if (Te > 0) atomicMin(&smin, Te);
         }
-        i64* dst[6] = {ta_off, tg_off, gf_off, nullptr, tx_off, nullptr};
+        i64* dst[6] = {ta_off, tg_off, gf_off, nullptr, nullptr, nullptr};
         if (in_rows) {
             if (ok) {
                 for (int k = 0; k < 6; k++) rows[k][b] = v[k];
             }
             __syncthreads();
             if (warp < 6) {
-                i64* to = warp == 0 ? ta_off : (warp == 1 ? tg_off : (warp == 2 ? gf_off : (warp == 4 ? tx_off : nullptr)));
+                i64* to = warp == 0 ? ta_off : (warp == 1 ? tg_off : (warp == 2 ? gf_off : nullptr));
                 const i64 total = warp_offsets(rows[warp], B, to);
                 if ((threadIdx.x & 31) == 0) carry[warp] = total;
             }
@@ -667,7 +665,6 @@ __global__ void __launch_bounds__(1024) k_off2(const int* __restrict__ state_off
         gf_off[B] = carry[2];
         gu_off[B] = carry[6];
         pu_off[B] = carry[7];
-        tx_off[B] = carry[4];
         hdr->score_floats = carry[4];
         hdr->T = T; hdr->B = B; hdr->F = F; hdr->E = E; hdr->S = S;
         hdr->state_floats = carry[0];
@@ -2502,7 +2499,7 @@ static int prepare_impl(const int32_t* edges, const float* weights, const int32_
                                at<int>(plan, L.end_l), at<i64>(plan, L.ta_off),
                                at<i64>(plan, L.tg_off), at<i64>(plan, L.gf_off),
                                at<i64>(plan, L.gu_off), at<i64>(plan, L.pu_off),
-                               at<i64>(plan, L.tx_off), at<i64>(plan, L.cost),
+                               at<i64>(plan, L.cost),
                                at<int>(plan, L.order), fast ? 1 : 0, hdr);
     if (E > 0 && !fast) {
         k_records<<<blocks(E), TB, 0, st>>>(
