@@ -24,9 +24,10 @@
 //
 // Arithmetic.  Scores grow with t (~2e4 at T=1500, one ulp = 2e-3), and a sum of two of them rounded to
 // that grid, as the reference forms it, shows in the posteriors:
-//   * the sweeps' log-sums are formed in scaled numbers (to_scaled): one relative rounding of 2^-24 per
-//     operation, whatever the accumulated score.  A stored state score is the natural negative log, rounded
-//     once; it is closer to the exact value than the reference's.
+//   * the sweeps' log-sums are formed in scaled numbers (scaled.h): a step rounds to about 2^-23 of the frame's
+//     own score, or of the sum where that is below one, whatever the accumulated score.  A stored state score is
+//     the natural negative log, rounded once; it is closer to the exact value than the reference's.
+//     (Sweeps of automata with several states per thread add logarithms, as the reference does.)
 //   * prob_add is fbw_op.cu:39-48 in meaning: min(a,b) - log1p(exp(-|a-b|)), +inf where both are +inf,
 //     rounded once to the grid of the result (see prob_add below for how the logarithm is formed).
 //   * an edge score is ((alpha + weight) + score) + beta (fbw_op.cu:93-99).
@@ -36,6 +37,7 @@
 
 #include "fbw_b200.h"
 #include "host_fill.h"
+#include "scaled.h"
 
 #include <cuda_runtime.h>
 #include <math_constants.h>
@@ -218,41 +220,6 @@ __device__ __forceinline__ float prob_add_live(float acc, float x) {
     if (x == CUDART_INF_F) return acc;
     if (acc == CUDART_INF_F) return prob_first(x);
     return prob_add(acc, x);
-}
-
-// Scaled numbers: x.x * 2^-x.y with x.y a whole number, +inf for zero (a dead state or edge).  The
-// exponent is a float so that +inf needs no special case and scores of any magnitude fit (above 2^24 its
-// spacing exceeds one, as the spacing of a score of that magnitude does).
-//
-// exp(-s) of a negative log score: s * log2(e) is split into the nearest whole number and a remainder,
-// formed with fused multiply-adds and log2(e) in two parts, so the mantissa (0.70 .. 1.42) carries the
-// score's own rounding and the exponential's (2^-22.5) only.  +inf and NaN give zero; finite scores beyond
-// the exponent's range saturate and stay finite.
-__device__ __forceinline__ float2 to_scaled(float s) {
-    const float c = rintf(fminf(fmaxf(s * 1.44269502f, -3.4e38f), 3.4e38f));
-    float r = fmaf(s, 1.44269502f, -c);
-    r = fmaf(s, 1.92596303e-8f, r);
-    r = fminf(fmaxf(r, -0.75f), 0.75f);
-    return make_float2(ex2_approx(-r), s < CUDART_INF_F ? c : CUDART_INF_F);
-}
-
-// 2^d for a whole number d <= 0; zero below 2^-126 and for NaN (the difference of two +inf)
-__device__ __forceinline__ float pow2_neg(float d) {
-    return __uint_as_float(__float_as_uint(fmaxf(d, -127.f) + 8388735.f) << 23);
-}
-
-// acc * 2^-c with the mantissa brought into [1,2); acc = 0 only where c = +inf
-__device__ __forceinline__ float2 normalised(float acc, float c) {
-    const unsigned u = __float_as_uint(acc);
-    return make_float2(__uint_as_float((u & 0x007fffffu) | 0x3f800000u),
-                       c - (__uint_as_float(0x4b000000u | (u >> 23)) - 8388735.f));
-}
-
-// the natural negative log of a scaled number (mantissa in [1,2)), rounded once
-__device__ __forceinline__ float from_scaled(float2 x) {
-    float l;
-    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(x.x));
-    return x.y < 3.4e38f ? fmaf(x.y, 0.693147181f, l * -0.693147181f) : x.y;
 }
 
 // largest b in [0,B) with off[b] <= u, given off[0] <= u < off[B]
@@ -1032,7 +999,7 @@ __global__ void __launch_bounds__(256) k_gather(RunArgs a) {
             }
             if (valid && c == nch - 1) {
                 for (int dd = Db + lane; dd < Dp; dd += 32) {
-                    if (gs) gs[(i64)t * Dp + dd] = make_float2(1.f, CUDART_INF_F);
+                    if (gs) gs[(i64)t * Dp + dd] = make_float2(0.f, CUDART_INF_F);
                     else if (!a.gathered_by_host) gf[(i64)t * Dp + dd] = 0.f;
                 }
             }
