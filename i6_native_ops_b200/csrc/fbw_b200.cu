@@ -30,10 +30,10 @@
 //     (Sweeps of automata with several states per thread add logarithms, as the reference does.)
 //   * prob_add is fbw_op.cu:39-48 in meaning: min(a,b) - log1p(exp(-|a-b|)), +inf where both are +inf,
 //     rounded once to the grid of the result (see prob_add below for how the logarithm is formed).
-//   * an edge score is ((alpha + weight) + score) + beta (fbw_op.cu:93-99).
-//   * class sums and the frame normaliser are scaled sums (minimum, sum of exp(minimum - x)) that stay
-//     differences until the end; the normaliser of sequences with few edges is the reference's left fold
-//     in ascending edge index (fbw_op.cu:115-118; see k_post).
+//   * an edge score is alpha + weight + score + beta (fbw_op.cu:93-99).  It, the class sums and the frame
+//     normaliser stay differences to the score of a good path until the end; sequences with few edges take
+//     the reference's order of operations and its left fold in ascending edge index (fbw_op.cu:115-118; see
+//     k_post).
 
 #include "fbw_b200.h"
 #include "host_fill.h"
@@ -1362,50 +1362,62 @@ __device__ __forceinline__ PostUnit post_unit(const RunArgs& a, i64 u) {
     return p;
 }
 
-// Sum of scaled terms (minimum, sum of exp(minimum - term)): adds s2 * exp(-m2) to s * exp(-m).  A term
-// that is +inf or NaN adds nothing.
+// Sums of negative logs: exp(-m) * (1 + s), m the smallest term and s the sum of exp(m - term) over the others.
+// Adds exp(-m2) * (1 + s2); a term that is +inf or NaN adds nothing.  The leading one stays outside s: where
+// one term holds nearly all of the probability, the log of the sum is as exact as s (see scaled.h).
 __device__ __forceinline__ void add_term(float& m, float& s, float m2, float s2) {
     const float e = ex2_approx(fabsf(m - m2) * -1.44269504f);  // 0 while the sum is empty (m = +inf)
     if (m2 < m) {
-        s = fmaf(s, e, s2);
+        s = fmaf(s, e, e) + s2;
         m = m2;
     } else if (m2 < CUDART_INF_F) {
-        s = fmaf(s2, e, s);
+        s += fmaf(s2, e, e);
     }
 }
 
 // Frame normalisers and class posteriors of one (sequence, 32-frame tile) per CTA step, lane = frame.
-//   x_e  = ((alpha_t(from) + w) + score_t(emission)) + beta_{t+1}(to)             (fbw_op.cu:93-100)
+//   x_e  = alpha_t(from) + w + score_t(emission) + beta_{t+1}(to)                 (fbw_op.cu:93-100)
 //   sum  = log-sum over all edges of x_e; sums[t,b] = 0 where no path exists        (fbw_op.cu:115-129)
 //   post = -log sum over the class's edges of exp(-(x_e - sum))                     (fbw_op.cu:131-153)
-// The edges come in class order (m_rec), an equal share of them per warp.  Every edge score is formed once,
-// in the reference's order of operations, and enters its class's running (minimum, scaled sum); finished
-// classes enter the frame's.  All values stay differences to a base near them until the normaliser is
-// known, so neither the class sums nor the normaliser are rounded to the grid of the scores (~1e4).
-// A class whose edges lie in the shares of several warps (a CTC blank has nearly half of all edges) is put
+// The edges come in class order (m_rec), an equal share of them per warp.  Every edge score is formed once
+// and enters its class's running sum (add_term); finished classes enter the frame's.  A class whose edges lie in
+// the shares of several warps (a CTC blank has nearly half of all edges) is put
 // aside as partial sums, head (the share's first class) and tail (its last), and merged by the warp in
 // whose share it starts.  The class values go where the class's score was (Gt, not needed any more); once
 // the normaliser is known they are read back and leave transposed, every frame's row of P contiguous.
 //
+// All scores are taken relative to a base, the score of the best path through the tile's second frame: a
+// sequence's sum is the same in every frame, so they are small numbers wherever a posterior is not, and neither
+// an edge score nor a class sum nor the normaliser is rounded to the grid of the accumulated scores (~1e4).  (With
+// the frame's first class as the base, which a model that is sure of its labels puts thousands above the sum,
+// posteriors were off by 1.2e-4 at a sum of 90, and by 1.5e-5 at one of 0.002.)
+//
 // Bound by the loads of state scores from L2 (two 128-byte lines per edge, one per class).  Before, the edge
 // scores of all frames went through memory (written once, read twice, with a serial fold over a sequence's
-// edges per frame between), in three kernels.
+// edges per frame between), in three kernels.  Four groups of 8 lattice sequences: 147, 662, 404 and 765 us
+// (207, 833, 573 and 932 with a base per warp, which every class then had to look up); 32 monophone sequences
+// 23 us (30).
 //
-// Sequences of at most kFoldEdges edges take the frame's sum as the reference forms it, a left fold in
-// ascending edge index rounded to the grid of the scores at every step (fbw_op.cu:115-118), over the edges
-// within e^-kFoldReach of the best: a smaller term changes no sum of that grid.  Such a fold loses the small
+// Sequences of at most kFoldEdges edges take the edge scores and the frame's sum as the reference forms them:
+// ((alpha + w) + score) + beta, and a left fold in ascending edge index rounded to the grid of the scores at every
+// step (fbw_op.cu:115-118), over the edges
+// within e^-kFoldReach of the best: what it leaves out, at most kFoldEdges * e^-kFoldReach = 2.6e-7, is below half a
+// spacing of a sum from kFoldCut on; smaller sums (a model that is sure of its labels) take every edge that
+// has a probability at all.  Such a fold loses the small
 // terms one by one, and posteriors come out up to 2e-4 too large (magnitude 1e3) as the reference's do; for
 // these sizes the results stay those of the reference and the fold is short (one warp, ~30 ns an edge).  For
-// longer lists the fold would be the longest part of the pass, and the scaled sum, which has no such
+// longer lists the fold would be the longest part of the pass, and the sum of classes, which has no such
 // error, takes its place.
 constexpr int   kPostWarps = 8;
 constexpr int   kFoldEdges = 128;
 constexpr float kFoldReach = 20.f;
+constexpr float kFoldCut   = 8.f;
 __global__ void __launch_bounds__(32 * kPostWarps, 3) k_post(RunArgs a) {
     constexpr int W = kPostWarps;
     __shared__ float stage[W][kTile][kTile + 1];
-    __shared__ float hm[W][kTile], hs[W][kTile], tm[W][kTile], ts[W][kTile], bw[W][kTile], fm[W][kTile], fs[W][kTile];
-    __shared__ int hslot[W], tslot[W], owned[W];
+    __shared__ float hm[W][kTile], hs[W][kTile], tm[W][kTile], ts[W][kTile], fm[W][kTile], fs[W][kTile];
+    __shared__ int hslot[W], tslot[W];
+    __shared__ float low[W];
     __shared__ unsigned short kept[W][kFoldEdges / W + 1];
     __shared__ int nkept[W];
     extern __shared__ float xs[];  // edge scores [position][frame] of a sequence of at most kFoldEdges edges
@@ -1423,95 +1435,53 @@ __global__ void __launch_bounds__(32 * kPostWarps, 3) k_post(RunArgs a) {
         float* Gb = a.Gt + a.tg_off[p.b] + (i64)p.k * p.Db * kTile + lane;
         const int4* __restrict__ rec = a.m_rec + p.e0;
         const bool fold = p.Eb <= kFoldEdges;
+        const int i0 = (int)((i64)warp * p.Eb / W), i1 = (int)((i64)(warp + 1) * p.Eb / W);  // this warp's share
 
-        // ---- classes of this warp's share of the edges ----
-        const int i0 = (int)((i64)warp * p.Eb / W), i1 = (int)((i64)(warp + 1) * p.Eb / W);
-        float base = CUDART_INF_F;                   // what this warp's class values are relative to
-        float nm = CUDART_INF_F, ns = 0.f;           // the share's part of the frame's sum
-        float cm = CUDART_INF_F, cs = 0.f;           // the running class
-        int   cur = -1, cnt = 0, head = -1, tail = -1;
-        auto store_class = [&](int slot, float m, float s, bool single) {
-            if (base == CUDART_INF_F && m < CUDART_INF_F) base = m;
-            const float v = (m - base) - (single ? 0.f : logf(s));
-            Gb[slot * kTile] = m == CUDART_INF_F ? CUDART_INF_F : v;
-        };
-        auto finish_class = [&]() {
-            add_term(nm, ns, cm, cs);
-            if (head < 0) {
-                head = cur;
-                hm[warp][lane] = cm;
-                hs[warp][lane] = cs;
-            } else {
-                store_class(cur, cm, cs, cnt == 1);
-            }
-        };
-        int4 rn[kPostBatch];  // the next batch's records: their loads go on beside the scores' loads
+        // use(record, alpha, score, beta) for the edges of the share, their lines loaded kPostBatch edges at a time
+        auto edges = [&](auto&& use) {
+            if (i0 >= i1) return;
+            int4 rn[kPostBatch];  // the next batch's records: their loads go on beside the scores' loads
 #pragma unroll
-        for (int j = 0; j < kPostBatch; j++) rn[j] = i0 < i1 ? __ldg(rec + min(i0 + j, i1 - 1)) : make_int4(0, 0, 0, 0);
-        for (int i = i0; i < i1; i += kPostBatch) {
-            int4  r[kPostBatch];
-            float al[kPostBatch], be[kPostBatch], g[kPostBatch];
+            for (int j = 0; j < kPostBatch; j++) rn[j] = __ldg(rec + min(i0 + j, i1 - 1));
+            for (int i = i0; i < i1; i += kPostBatch) {
+                int4  r[kPostBatch];
+                float al[kPostBatch], be[kPostBatch], g[kPostBatch];
 #pragma unroll
-            for (int j = 0; j < kPostBatch; j++) {
-                r[j]  = rn[j];
-                rn[j] = __ldg(rec + min(i + kPostBatch + j, i1 - 1));
-            }
+                for (int j = 0; j < kPostBatch; j++) {
+                    r[j]  = rn[j];
+                    rn[j] = __ldg(rec + min(i + kPostBatch + j, i1 - 1));
+                }
 #pragma unroll
-            for (int j = 0; j < kPostBatch; j++) {
-                al[j] = Ab[(r[j].x & 0xffff) * kTile];
-                be[j] = Bb[((unsigned)r[j].x >> 16) * kTile];
-                g[j]  = Gb[r[j].z * kTile];
-            }
+                for (int j = 0; j < kPostBatch; j++) {
+                    al[j] = Ab[(r[j].x & 0xffff) * kTile];
+                    be[j] = Bb[((unsigned)r[j].x >> 16) * kTile];
+                    g[j]  = Gb[r[j].z * kTile];
+                }
 #pragma unroll
-            for (int j = 0; j < kPostBatch; j++) {
-                if (i + j >= i1) continue;  // uniform
-                const float v = ((al[j] + __int_as_float(r[j].w)) + g[j]) + be[j];
-                const float x = valid ? v : CUDART_INF_F;
-                if (fold) xs[r[j].y * kTile + lane] = x;
-                if (r[j].z != cur) {  // uniform: a new class starts
-                    if (cur >= 0) finish_class();
-                    cur = r[j].z;
-                    cnt = 1;
-                    cm  = x;
-                    cs  = 1.f;
-                } else {
-                    add_term(cm, cs, x, 1.f);
-                    cnt++;
+                for (int j = 0; j < kPostBatch; j++) {
+                    if (i + j < i1) use(r[j], al[j], g[j], be[j]);  // uniform
                 }
             }
-        }
-        if (cur >= 0) {  // the share's last class may go on in the next warp's share
-            add_term(nm, ns, cm, cs);
-            if (head < 0) {
-                head = cur;
-                hm[warp][lane] = cm;
-                hs[warp][lane] = cs;
-            } else {
-                tail = cur;
-                tm[warp][lane] = cm;
-                ts[warp][lane] = cs;
-            }
-        }
-        fm[warp][lane] = nm;
-        fs[warp][lane] = ns;
-        if (lane == 0) {
-            hslot[warp] = head;
-            tslot[warp] = tail;
-        }
-        __syncthreads();
+        };
 
-        // ---- the normaliser, and the classes that several warps share ----
-        nm = CUDART_INF_F;
-        ns = 0.f;
-#pragma unroll
-        for (int w = 0; w < W; w++) add_term(nm, ns, fm[w][lane], fs[w][lane]);
-        float logn = logf(ns);
+        float nm = CUDART_INF_F, ns = 0.f;  // the frame's sum
+        float base = 0.f;
         if (fold) {
-            // the edges (ascending) that can move the sum of some frame of the tile: within kFoldReach of its
-            // smallest score
+            edges([&](int4 r, float al, float g, float be) {
+                const float v = ((al + __int_as_float(r.w)) + g) + be;
+                const float x = valid ? v : CUDART_INF_F;
+                xs[r.y * kTile + lane] = x;
+                nm = fminf(nm, x);
+            });
+            fm[warp][lane] = nm;
+            __syncthreads();
+#pragma unroll
+            for (int w = 0; w < W; w++) nm = fminf(nm, fm[w][lane]);
+            // the edges (ascending) that can move the sum of some frame of the tile
+            const float reach = fminf(nm + (fabsf(nm) >= kFoldCut ? kFoldReach : 104.f), 3.4e38f);
             int n = 0;
             for (int i = i0; i < i1; i++) {
-                if (__any_sync(0xffffffffu, xs[i * kTile + lane] <= fminf(nm + kFoldReach, 3.4e38f))) {
+                if (__any_sync(0xffffffffu, xs[i * kTile + lane] <= reach)) {
                     if (lane == 0) kept[warp][n] = (unsigned short)i;
                     n++;
                 }
@@ -1529,11 +1499,107 @@ __global__ void __launch_bounds__(32 * kPostWarps, 3) k_post(RunArgs a) {
             }
             __syncthreads();
             nm = fm[0][lane];
-            logn = 0.f;
+        } else {
+            // the best path through frame 1 of the tile: alpha of its states and beta, which is stored a frame
+            // earlier; a tile with one valid frame goes over the edges of that frame
+            const float* A0 = Ab - lane;
+            const float* B0 = Bb - lane;
+            float best = CUDART_INF_F;
+            if (p.k * kTile + 1 < p.Te) {
+#pragma unroll 4
+                for (int s = threadIdx.x; s < p.Sb; s += 32 * W) best = fminf(best, A0[s * kTile + 1] + B0[s * kTile]);
+            } else {
+                for (int i = threadIdx.x; i < p.Eb; i += 32 * W) {
+                    const int4 r = __ldg(rec + i);
+                    best = fminf(best, (A0[(r.x & 0xffff) * kTile] + B0[((unsigned)r.x >> 16) * kTile]) +
+                                           (__int_as_float(r.w) + (Gb - lane)[r.z * kTile]));
+                }
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) best = fminf(best, __shfl_xor_sync(0xffffffffu, best, o));
+            if (lane == 0) low[warp] = best;
+            __syncthreads();
+#pragma unroll
+            for (int w = 0; w < W; w++) best = fminf(best, low[w]);
+            base = best < CUDART_INF_F ? best : 0.f;  // +inf: no path, no finite score
         }
+
+        // ---- classes of this warp's share of the edges ----
+        float wm = CUDART_INF_F, ws = 0.f;           // the share's part of the frame's sum
+        float cm = CUDART_INF_F, cs = 0.f;           // the running class
+        int   cur = -1, cnt = 0, head = -1, tail = -1;
+        auto store_class = [&](int slot, float m, float s, bool single) {
+            Gb[slot * kTile] = m == CUDART_INF_F || single ? m : m - log1pf(s);
+        };
+        auto finish_class = [&]() {
+            add_term(wm, ws, cm, cs);
+            if (head < 0) {
+                head = cur;
+                hm[warp][lane] = cm;
+                hs[warp][lane] = cs;
+            } else {
+                store_class(cur, cm, cs, cnt == 1);
+            }
+        };
+        auto enter = [&](int slot, float x) {
+            if (slot != cur) {  // uniform: a new class starts
+                if (cur >= 0) finish_class();
+                cur = slot;
+                cnt = 1;
+                cm  = x;
+                cs  = 0.f;
+            } else {
+                add_term(cm, cs, x, 0.f);
+                cnt++;
+            }
+        };
+        if (fold) {  // the scores less the normaliser
+            for (int i = i0; i < i1; i++) {
+                const int4  r = __ldg(rec + i);
+                const float x = xs[r.y * kTile + lane];
+                enter(r.z, x < CUDART_INF_F ? x - nm : x);
+            }
+        } else {
+            edges([&](int4 r, float al, float g, float be) {
+                // alpha + beta and the exact remainder of its rounding (Knuth's two-sum); the difference to the
+                // base of a score near it is exact
+                const float q  = __int_as_float(r.w) + g;
+                const float h  = al + be, hb = h - al;
+                const float lo = (al - (h - hb)) + (be - hb);
+                const float x  = h < CUDART_INF_F ? (h - base) + (lo + q) : h + q;
+                enter(r.z, valid ? x : CUDART_INF_F);
+            });
+        }
+        if (cur >= 0) {  // the share's last class may go on in the next warp's share
+            add_term(wm, ws, cm, cs);
+            if (head < 0) {
+                head = cur;
+                hm[warp][lane] = cm;
+                hs[warp][lane] = cs;
+            } else {
+                tail = cur;
+                tm[warp][lane] = cm;
+                ts[warp][lane] = cs;
+            }
+        }
+        if (!fold) {
+            fm[warp][lane] = wm;
+            fs[warp][lane] = ws;
+        }
+        if (lane == 0) {
+            hslot[warp] = head;
+            tslot[warp] = tail;
+        }
+        __syncthreads();
+
+        // ---- the normaliser, and the classes that several warps share ----
+        if (!fold) {
+#pragma unroll
+            for (int w = 0; w < W; w++) add_term(nm, ns, fm[w][lane], fs[w][lane]);
+        }
+        const float logn = log1pf(ns);
         const bool  dead = !(nm < CUDART_INF_F);  // no path through this frame
-        if (warp == 0 && valid) a.sums[(i64)t * a.B + p.b] = dead ? 0.f : nm - logn;
-        int own = 0x7fffffff;  // first class whose value this warp writes
+        if (warp == 0 && valid) a.sums[(i64)t * a.B + p.b] = dead ? 0.f : base + (nm - logn);
         if (head >= 0) {
             int before = -1;  // the class that is running when this warp's share begins
             for (int w = warp - 1; w >= 0; w--) {
@@ -1555,30 +1621,19 @@ __global__ void __launch_bounds__(32 * kPostWarps, 3) k_post(RunArgs a) {
             if (starts && tail >= 0) store_class(head, hm[warp][lane], hs[warp][lane], false);
             if (starts && tail < 0) with_heads(head, hm[warp][lane], hs[warp][lane]);
             if (tail >= 0) with_heads(tail, tm[warp][lane], ts[warp][lane]);
-            if (starts) own = head;
-            else if (tail >= 0) own = head + 1;
         }
-        bw[warp][lane] = base;
-        if (lane == 0) owned[warp] = own;
         __syncthreads();
 
         // ---- posteriors, transposed: frame r of the tile gets its classes as one contiguous write ----
         float* __restrict__ Pb = a.P + a.gf_off[p.b];
         float (*st)[kTile + 1] = stage[warp];
+        const float norm = fold ? 0.f : nm;  // (the differences are already taken)
         for (int d0 = warp * kTile; d0 < p.Db; d0 += W * kTile) {
             const int nd = min(kTile, p.Db - d0);
-            int w = 0;
-            for (int q = 1; q < W; q++) w = owned[q] <= d0 ? q : w;
-            float shift = bw[w][lane] - nm;
 #pragma unroll 8
             for (int d = 0; d < nd; d++) {
                 const float x = Gb[(d0 + d) * kTile];
-                bool moved = false;
-                for (int q = w + 1; q < W; q++) {
-                    if (owned[q] == d0 + d) { w = q; moved = true; }
-                }
-                if (moved) shift = bw[w][lane] - nm;
-                st[d][lane] = dead || x == CUDART_INF_F ? CUDART_INF_F : (x + shift) + logn;
+                st[d][lane] = dead || x == CUDART_INF_F ? CUDART_INF_F : (x - norm) + logn;
             }
             __syncwarp();
             for (int r = 0; r < kTile; r++) {
