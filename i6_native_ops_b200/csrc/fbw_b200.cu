@@ -2013,14 +2013,18 @@ int sm_count() {
 }
 
 // Raise a kernel's dynamic shared-memory limit to `smem` bytes unless an earlier launch on this
-// device already raised it that far (`granted` is the per-device record of one kernel).
+// device already raised it that far (`granted` is the per-device record of one kernel).  Every size is
+// asked for: without it a launch may use 48 KB less the kernel's static shared memory, which differs from
+// kernel to kernel.  The lock keeps a smaller request of another thread from replacing a larger one.
 template <typename Kernel>
-cudaError_t grant_smem(Kernel kernel, std::atomic<int>* granted, size_t smem, size_t fixed = 0) {
-    if (smem + fixed <= 48 * 1024) return cudaSuccess;  // (fixed: the kernel's static shared memory)
+cudaError_t grant_smem(Kernel kernel, std::atomic<int>* granted, size_t smem) {
     const int dev = current_device();
+    if ((size_t)granted[dev].load(std::memory_order_acquire) >= smem) return cudaSuccess;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
     if ((size_t)granted[dev].load(std::memory_order_relaxed) >= smem) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) granted[dev].store((int)smem, std::memory_order_relaxed);
+    if (e == cudaSuccess) granted[dev].store((int)smem, std::memory_order_release);
     return e;
 }
 
@@ -2338,7 +2342,7 @@ int launch_group(RunArgs a, int r0, int r1, i64 ms, i64 me, i64 md, const fbw_b2
         const int grid = (int)(units < (i64)sms * 6 ? units : (i64)sms * 6);
         const size_t xs = sizeof(float) * kTile * (size_t)(me < kFoldEdges ? me : kFoldEdges);
         static std::atomic<int> granted[kMaxDevices];
-        CUDA_OK(grant_smem(k_post, granted, sizeof(float) * kTile * kFoldEdges, 42 * 1024));
+        CUDA_OK(grant_smem(k_post, granted, sizeof(float) * kTile * kFoldEdges));
         k_post<<<grid > 0 ? grid : 1, 32 * kPostWarps, xs, st>>>(a);
         COUNT_LAUNCH(1);
     }
