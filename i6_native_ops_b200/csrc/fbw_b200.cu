@@ -900,7 +900,9 @@ struct RunArgs {
     // Time chunks: the sweeps advance chunk_steps frames per chunk from both ends of a sequence; a
     // launch handles the chunks [c_lo, c_hi).  One chunk covering everything is the plain case.
     int c_lo, c_hi, chunk_steps;
-    float* carry;  // state vectors handed from one sweep chunk to the next, float or float2 [2 * state][direction]
+    // state vectors handed from one sweep chunk to the next: four floats a state, of which a sequence uses a float or
+    // a float2 per state and direction
+    float* carry;
     // 1: the wrapper's passes are folded in -- `am` is log_probs (B,T,F) (sign and layout of the
     // caller's tensor, i6_native_ops/fbw/__init__.py:66) and `out` receives the gradient with respect
     // to it, -posterior in (B,T,F) with zeros elsewhere (what __init__.py:41-44 and autograd produce)
@@ -1181,7 +1183,7 @@ __global__ void __launch_bounds__(1024) k_sweep(RunArgs a, int smax, int dpmax, 
     const int j0 = a.c_lo * a.chunk_steps;
     const int j1 = (int)min((i64)a.c_hi * a.chunk_steps, (i64)Te);
     if (j0 >= Te) return;
-    float* __restrict__ carry = a.carry + 2 * (i64)s0 + (fwd ? 0 : Sb);
+    float* __restrict__ carry = a.carry + 4 * (i64)s0 + (fwd ? 0 : Sb);
     {
         const int seed = fwd ? a.start_l[b] : a.end_l[b];
         float* r0 = srow(j0, t_first + step * j0);
@@ -2258,29 +2260,133 @@ bool output_in_two_steps(const fbw_b200_summary& s, i64 ms, i64 me, i64 md) {
     return fill_ms >= 1.3 * sweep_ms;
 }
 
-// gather -> sweep -> posterior -> expand for the sequences of ranks [r0, r1) on stream st.
-// ms/me/md: largest state, edge and slot counts in the range (they size the sweep launch).
-enum { kDoGather = 1, kDoSweep = 2, kDoPost = 4, kDoExpand = 8, kDoAll = 15, kDoPatch = 16 };
+// Which sweep every base group (an eighth of the cost order) takes: scaled numbers or logarithms, which differ
+// in rounding, and on clusters of how many CTAs.  It follows from the summary alone -- from the groups in which
+// fbw_b200_run would launch the batch into device memory -- and holds for every schedule (groups, time chunks,
+// one launch, the library's own scratch), so that all entry points give the same bits.
+struct SweepPlan {
+    int  groups;    // groups of that schedule
+    bool two_step;  // and whether it writes the output in two steps (given a destination that allows it)
+    bool clustered;
+    bool scaled[FBW_B200_GROUPS];
+    int  cs[FBW_B200_GROUPS];
+};
+int base_rank(const fbw_b200_summary& s, int q) { return (int)(((i64)q * s.B) / FBW_B200_GROUPS); }
 
-// `what` selects the stages to launch (the time-chunked pipeline launches them on different streams)
-int launch_group(RunArgs a, int r0, int r1, i64 ms, i64 me, i64 md, const fbw_b200_summary& s,
-                 cudaStream_t st, cudaEvent_t* ev, int what = kDoAll, int cs = 1) {
-    const int sms = sm_count();
-    const int nb  = r1 - r0;
+SweepPlan sweep_plan(const fbw_b200_summary& s) {
+    SweepPlan p;
+    memset(&p, 0, sizeof(p));
+    i64 ms, me, md;
+    plan_maxima(s, ms, me, md);
+    // Output in two steps: four groups, most expensive first.  Large calls that can write their output
+    // that way run as groups whatever their batch size: with the background written during the sweeps
+    // the group schedule beats the time-chunk pipeline also for few sequences (triphone, ms per call,
+    // chunks against groups: 8 sequences 1.35 / 1.28, 16: 1.44 / 1.39, 32: 1.79 / 1.70, 48: 2.21 / 1.97;
+    // BPE-CTC 32 sequences 0.68 / 0.61).
+    const bool groups_forced = getenv("FBW_B200_NUM_GROUPS") != nullptr;
+    const bool can_two_step  = output_in_two_steps(s, ms, me, md);
+    int G = choose_groups(s);
+    if (can_two_step && G == 1 && !groups_forced && s.B >= 4 && (double)s.T * (double)s.B * (double)s.F >= 1.0e8) G = 4;
+    p.two_step = G > 1 && can_two_step;
+    if (p.two_step && G == 8 && !groups_forced) G = 4;
+    p.groups = G;
+    int spare;
+    if (G == 1) {
+        spare = sm_count() - 2 * (int)s.B;
+    } else {
+        // Clusters for the groups of the largest automata, most expensive group first, while the
+        // call's sweep CTAs stay below 1.65 per SM (the CTAs of short sequences leave early;
+        // measured on 64 lattice sequences: 24.6 ms without clusters, 18.6 ms filling the idle SMs
+        // only, 15.0 ms with a bound of 1.5, 14.4 ms with 1.65, 14.6 ms with 1.8).
+        static double oversub = -1.0;
+        if (oversub < 0) { const char* e = getenv("FBW_B200_CLUSTER_OVERSUB"); oversub = e ? atof(e) : 0.65; }
+        spare = (int)(sm_count() * (1.0 + oversub)) - 2 * (int)s.B;
+        // up to four sweep CTAs per SM the most expensive sequences still get clusters worth 15 %
+        // more CTAs: their sweeps, not the amount of work, end the call (128 lattice sequences:
+        // 26.0 -> 17.7 ms; 256: 31.9 -> 30.6 ms; 512 sequences are better off without: 56 -> 59 ms)
+        static double share = -1.0;
+        if (share < 0) { const char* e = getenv("FBW_B200_CLUSTER_SHARE"); share = e ? atof(e) : 0.15; }
+        if (2 * s.B <= 4 * (i64)sm_count() && spare < (int)(share * 2 * (double)s.B)) {
+            spare = (int)(share * 2 * (double)s.B);
+        }
+    }
+    const int per = FBW_B200_GROUPS / G;
+    for (int q0 = 0; q0 < FBW_B200_GROUPS; q0 += per) {
+        i64 gs = 0, ge = 0, gd = 0;
+        for (int q = q0; q < q0 + per; q++) {
+            gs = s.group_max_states[q] > gs ? s.group_max_states[q] : gs;
+            ge = s.group_max_edges[q] > ge ? s.group_max_edges[q] : ge;
+            gd = s.group_max_slots[q] > gd ? s.group_max_slots[q] : gd;
+        }
+        const int items = 2 * (base_rank(s, q0 + per) - base_rank(s, q0));
+        // (the background of an output in two steps is written by the sweeps of one CTA)
+        const int cs = p.two_step ? 1 : sweep_cluster_size(gs, items, &spare);
+        const bool scaled = scaled_shape(gs, ge, gd, s.max_degree, cs).found;
+        p.clustered = p.clustered || cs > 1;
+        for (int q = q0; q < q0 + per; q++) {
+            p.cs[q]     = cs;
+            p.scaled[q] = scaled;
+        }
+    }
+    return p;
+}
+
+// The ranks [r0, r1) as runs of base groups that one sweep launch can serve
+struct SweepRun {
+    int  r0, r1, cs;
+    bool scaled;
+    i64  ms, me, md;
+};
+int sweep_runs(const fbw_b200_summary& s, const SweepPlan& p, int r0, int r1, SweepRun* runs) {
+    int n = 0;
+    for (int q = 0; q < FBW_B200_GROUPS; q++) {
+        SweepRun r;
+        r.r0 = base_rank(s, q) > r0 ? base_rank(s, q) : r0;
+        r.r1 = base_rank(s, q + 1) < r1 ? base_rank(s, q + 1) : r1;
+        if (r.r1 <= r.r0) continue;
+        r.cs = p.cs[q];
+        r.scaled = p.scaled[q];
+        r.ms = s.group_max_states[q];
+        r.me = s.group_max_edges[q];
+        r.md = s.group_max_slots[q];
+        if (n > 0 && runs[n - 1].cs == r.cs && runs[n - 1].scaled == r.scaled) {
+            SweepRun u = runs[n - 1];
+            u.r1 = r.r1;
+            u.ms = r.ms > u.ms ? r.ms : u.ms;
+            u.me = r.me > u.me ? r.me : u.me;
+            u.md = r.md > u.md ? r.md : u.md;
+            if (!u.scaled || scaled_shape(u.ms, u.me, u.md, s.max_degree, u.cs).found) {
+                runs[n - 1] = u;
+                continue;
+            }
+        }
+        runs[n++] = r;
+    }
+    return n;
+}
+
+// the compact score arrays of the ranks [r0, r1), at most md classes a sequence
+int launch_gather(RunArgs a, int r0, int r1, i64 md, const fbw_b200_summary& s, cudaStream_t st) {
+    if (s.gather_units <= 0 || md <= 0) return FBW_B200_OK;
     a.r0 = r0;
     a.r1 = r1;
-    const i64 tiles = (s.max_len + kTile - 1) / kTile;
-    const ScaledShape sc = scaled_shape(ms, me, md, s.max_degree, cs);
-    if (!sc.found || cs > 1) a.Gs = nullptr;  // those sweeps read the raw scores
-    if (ev) CUDA_OK(cudaEventRecord(ev[0], st));
-    if ((what & kDoGather) && s.gather_units > 0 && md > 0) {
-        i64 want = tiles * nb * ((md + kGatherSlots - 1) / kGatherSlots);
-        int grid = (int)(want < (i64)sms * 6 ? want : (i64)sms * 6);
-        k_gather<<<grid > 0 ? grid : 1, 256, 0, st>>>(a);
-        COUNT_LAUNCH(1);
-    }
-    if (ev) CUDA_OK(cudaEventRecord(ev[1], st));
-    if ((what & kDoSweep) && s.max_len > 0 && sc.found) {
+    const i64 most = (i64)sm_count() * 6;
+    const i64 want = (s.max_len + kTile - 1) / kTile * (r1 - r0) * ((md + kGatherSlots - 1) / kGatherSlots);
+    const int grid = (int)(want < most ? want : most);
+    k_gather<<<grid > 0 ? grid : 1, 256, 0, st>>>(a);
+    COUNT_LAUNCH(1);
+    return FBW_B200_OK;
+}
+
+// the sweeps of one run of groups
+int launch_sweeps(RunArgs a, const SweepRun& r, const fbw_b200_summary& s, cudaStream_t st) {
+    const int nb = r.r1 - r.r0;
+    const int cs = r.cs;
+    const i64 ms = r.ms, me = r.me, md = r.md;
+    a.r0 = r.r0;
+    a.r1 = r.r1;
+    if (r.scaled) {
+        const ScaledShape sc = scaled_shape(ms, me, md, s.max_degree, cs);
         int rc;
         if (cs > 1) {
             rc = launch_cluster(a, sc, 2 * nb, st);
@@ -2296,10 +2402,10 @@ int launch_group(RunArgs a, int r0, int r1, i64 ms, i64 me, i64 md, const fbw_b2
                               sc.nt + (a.next_row != nullptr ? 32 : 0), smem, st);
         }
         if (rc != FBW_B200_OK) return rc;
-    } else if ((what & kDoSweep) && s.max_len > 0 && cs > 1 && cluster_shape(ms, me, md, cs < 4 ? cs : 4).found) {
+    } else if (cs > 1 && cluster_shape(ms, me, md, cs < 4 ? cs : 4).found) {
         const int rc = launch_sweepc(a, cluster_shape(ms, me, md, cs < 4 ? cs : 4), 2 * nb, st);
         if (rc != FBW_B200_OK) return rc;
-    } else if ((what & kDoSweep) && s.max_len > 0) {
+    } else {
         const SweepShape c = sweep_shape(ms, me, md);
         if (!c.found) return FBW_B200_TOO_LARGE;
         const int smax = c.smax, dpmax = c.dpmax, nt = c.nt, ring = c.ring, tiled = c.tiled;
@@ -2334,6 +2440,35 @@ int launch_group(RunArgs a, int r0, int r1, i64 ms, i64 me, i64 md, const fbw_b2
             }
         }
 #undef SWEEP_CASE
+        if (rc != FBW_B200_OK) return rc;
+    }
+    return FBW_B200_OK;
+}
+
+// gather -> sweep -> posterior -> expand for the sequences of ranks [r0, r1) on stream st.
+// me: largest edge count in the range.
+enum { kDoGather = 1, kDoSweep = 2, kDoPost = 4, kDoExpand = 8, kDoAll = 15, kDoPatch = 16 };
+
+// `what` selects the stages to launch (the time-chunked pipeline launches them on different streams)
+int launch_group(RunArgs a, int r0, int r1, i64 me, const fbw_b200_summary& s, const SweepPlan& plan,
+                 cudaStream_t st, cudaEvent_t* ev, int what = kDoAll) {
+    const int sms = sm_count();
+    const int nb  = r1 - r0;
+    a.r0 = r0;
+    a.r1 = r1;
+    const i64 tiles = (s.max_len + kTile - 1) / kTile;
+    SweepRun runs[FBW_B200_GROUPS];
+    const int nruns = sweep_runs(s, plan, r0, r1, runs);
+    if (ev) CUDA_OK(cudaEventRecord(ev[0], st));
+    for (int i = 0; (what & kDoGather) && i < nruns; i++) {
+        RunArgs g = a;
+        if (!runs[i].scaled || runs[i].cs > 1) g.Gs = nullptr;  // those sweeps read the raw scores
+        const int rc = launch_gather(g, runs[i].r0, runs[i].r1, runs[i].md, s, st);
+        if (rc != FBW_B200_OK) return rc;
+    }
+    if (ev) CUDA_OK(cudaEventRecord(ev[1], st));
+    for (int i = 0; (what & kDoSweep) && s.max_len > 0 && i < nruns; i++) {
+        const int rc = launch_sweeps(a, runs[i], s, st);
         if (rc != FBW_B200_OK) return rc;
     }
     if (ev) CUDA_OK(cudaEventRecord(ev[2], st));
@@ -2686,25 +2821,19 @@ static int run_impl(const void* plan, const fbw_b200_summary* summary, const flo
             host_scores = false;  // from here on the call is one whose scores are on the device
         }
     }
-    int G = ev ? 1 : choose_groups(s);
-    if (G > 1 && host_scores && !(s.max_edges >= 2048 && (double)s.max_edges * (double)s.B >= 1.8 * (double)s.E)) G = 1;
-    if (host_patch) G = 1;  // the host's row order follows the time chunks
     i64 ms, me, md;
     plan_maxima(s, ms, me, md);
-    // Output in two steps: four groups, most expensive first.  Large calls that can write their output
-    // that way run as groups whatever their batch size: with the background written during the sweeps
-    // the group schedule beats the time-chunk pipeline also for few sequences (triphone, ms per call,
-    // chunks against groups: 8 sequences 1.35 / 1.28, 16: 1.44 / 1.39, 32: 1.79 / 1.70, 48: 2.21 / 1.97;
-    // BPE-CTC 32 sequences 0.68 / 0.61).
+    const SweepPlan sweeps = sweep_plan(s);
     const bool groups_forced = getenv("FBW_B200_NUM_GROUPS") != nullptr;
-    const bool can_two_step = !ev && fused != 2 && !a.out_plain && (((uintptr_t)out & 31) == 0) &&
-                              output_in_two_steps(s, ms, me, md);
-    if (can_two_step && G == 1 && !groups_forced && !host_scores && !host_patch && s.B >= 4 &&
-        (double)s.T * (double)s.B * (double)s.F >= 1.0e8) {
-        G = 4;
+    // the schedule of sweep_plan, unless the scores' or the result's place asks for another one
+    bool two_step = sweeps.two_step && !a.out_plain && (((uintptr_t)out & 31) == 0);
+    int  G = two_step ? sweeps.groups : choose_groups(s);
+    if (host_scores && (choose_groups(s) == 1 ||
+                        !(s.max_edges >= 2048 && (double)s.max_edges * (double)s.B >= 1.8 * (double)s.E))) {
+        G = 1;
     }
-    const bool two_step = G > 1 && can_two_step;
-    if (two_step && G == 8 && !groups_forced) G = 4;
+    if (ev || host_patch) G = 1;  // one event per stage; the host's row order follows the time chunks
+    two_step = two_step && G > 1;
     const int C = (ev || G > 1) ? 1 : choose_chunks(s);
     // every launch shape is checked before anything is enqueued, so that a call that cannot run
     // fails before it has forked onto the auxiliary streams
@@ -2722,50 +2851,18 @@ static int run_impl(const void* plan, const fbw_b200_summary* summary, const flo
         // expensive groups are still sweeping (FBW_B200_GROUP_ORDER=0: most expensive first)
         static int reverse = -1;
         if (reverse < 0) { const char* e = getenv("FBW_B200_GROUP_ORDER"); reverse = e ? atoi(e) : 1; }
-        // Clusters for the groups of the largest automata, most expensive group first, while the
-        // call's sweep CTAs stay below 1.65 per SM (the CTAs of short sequences leave early;
-        // measured on 64 lattice sequences: 24.6 ms without clusters, 18.6 ms filling the idle SMs
-        // only, 15.0 ms with a bound of 1.5, 14.4 ms with 1.65, 14.6 ms with 1.8).
-        int group_cs[FBW_B200_GROUPS];
-        bool clustered = false;
-        {
-            static double oversub = -1.0;
-            if (oversub < 0) { const char* e = getenv("FBW_B200_CLUSTER_OVERSUB"); oversub = e ? atof(e) : 0.65; }
-            int spare = (int)(sm_count() * (1.0 + oversub)) - 2 * (int)s.B;
-            // up to four sweep CTAs per SM the most expensive sequences still get clusters worth 15 %
-            // more CTAs: their sweeps, not the amount of work, end the call (128 lattice sequences:
-            // 26.0 -> 17.7 ms; 256: 31.9 -> 30.6 ms; 512 sequences are better off without: 56 -> 59 ms)
-            static double share = -1.0;
-            if (share < 0) { const char* e = getenv("FBW_B200_CLUSTER_SHARE"); share = e ? atof(e) : 0.15; }
-            if (2 * s.B <= 4 * (i64)sm_count() && spare < (int)(share * 2 * (double)s.B)) {
-                spare = (int)(share * 2 * (double)s.B);
-            }
-            for (int g = 0; g < G; g++) {
-                const int r0 = (int)(((i64)(g * per) * s.B) / FBW_B200_GROUPS);
-                const int r1 = (int)(((i64)((g + 1) * per) * s.B) / FBW_B200_GROUPS);
-                i64 gs_ = 0;
-                for (int q = g * per; q < (g + 1) * per; q++) gs_ = s.group_max_states[q] > gs_ ? s.group_max_states[q] : gs_;
-                group_cs[g] = sweep_cluster_size(gs_, 2 * (r1 - r0), &spare);
-                clustered = clustered || group_cs[g] > 1;
-            }
-        }
         // with clusters the long sequences are the critical path: they start first
-        const bool cheapest_first = reverse && !clustered && !two_step;
-        struct GroupRun { int r0, r1, cs; i64 ms, me, md; cudaStream_t st; } runs[FBW_B200_GROUPS];
+        const bool cheapest_first = reverse && !sweeps.clustered && !two_step;
+        struct GroupRun { int r0, r1; i64 me; cudaStream_t st; } runs[FBW_B200_GROUPS];
         int nruns = 0;
         for (int gi = 0; gi < G; gi++) {
             const int g = cheapest_first ? G - 1 - gi : gi;
             GroupRun r;
-            r.r0 = (int)(((i64)(g * per) * s.B) / FBW_B200_GROUPS);
-            r.r1 = (int)(((i64)((g + 1) * per) * s.B) / FBW_B200_GROUPS);
+            r.r0 = base_rank(s, g * per);
+            r.r1 = base_rank(s, (g + 1) * per);
             if (r.r1 <= r.r0) continue;
-            r.ms = r.me = r.md = 0;
-            for (int q = g * per; q < (g + 1) * per; q++) {
-                r.ms = s.group_max_states[q] > r.ms ? s.group_max_states[q] : r.ms;
-                r.me = s.group_max_edges[q] > r.me ? s.group_max_edges[q] : r.me;
-                r.md = s.group_max_slots[q] > r.md ? s.group_max_slots[q] : r.md;
-            }
-            r.cs = group_cs[g];
+            r.me = 0;
+            for (int q = g * per; q < (g + 1) * per; q++) r.me = s.group_max_edges[q] > r.me ? s.group_max_edges[q] : r.me;
             r.st = nruns == 0 ? st : pool->aux[nruns];
             runs[nruns++] = r;
         }
@@ -2792,8 +2889,8 @@ static int run_impl(const void* plan, const fbw_b200_summary* summary, const flo
                 // 1.29 ms with 2 KB pieces, 1.34 with 8 KB).
                 ag.fill_piece = 2 * s.B > (i64)sm_count() ? 512 : kFillFloats;
             }
-            int rc = launch_group(ag, r.r0, r.r1, r.ms, r.me, r.md, s, r.st, nullptr,
-                                  two_step ? (kDoGather | kDoSweep | kDoPost | kDoPatch) : kStages, r.cs);
+            int rc = launch_group(ag, r.r0, r.r1, r.me, s, sweeps, r.st, nullptr,
+                                  two_step ? (kDoGather | kDoSweep | kDoPost | kDoPatch) : kStages);
             if (i > 0 && (cudaEventRecord(pool->join[i], r.st) != cudaSuccess ||
                           cudaStreamWaitEvent(st, pool->join[i], 0) != cudaSuccess)) {
                 rc = rc != FBW_B200_OK ? rc : FBW_B200_CUDA_ERROR;
@@ -2818,12 +2915,10 @@ static int run_impl(const void* plan, const fbw_b200_summary* summary, const flo
             if (e != cudaSuccess && rc_forked == FBW_B200_OK) rc_forked = FBW_B200_CUDA_ERROR;
             return rc_forked == FBW_B200_OK;
         };
-        int spare = sm_count() - 2 * (int)s.B;
-        const int cs_all = sweep_cluster_size(ms, 2 * (int)s.B, &spare);
         auto stage = [&](int c, cudaStream_t on, int what) {
             a.c_lo = c;
             a.c_hi = c + 1;
-            const int rc = launch_group(a, 0, (int)s.B, ms, me, md, s, on, nullptr, what, cs_all);
+            const int rc = launch_group(a, 0, (int)s.B, me, s, sweeps, on, nullptr, what);
             if (rc != FBW_B200_OK && rc_forked == FBW_B200_OK) rc_forked = rc;
             return rc_forked == FBW_B200_OK;
         };
@@ -2902,9 +2997,7 @@ static int run_impl(const void* plan, const fbw_b200_summary* summary, const flo
             }
         }
     } else {
-        int spare = sm_count() - 2 * (int)s.B;
-        int rc = launch_group(a, 0, (int)s.B, ms, me, md, s, st, ev, kStages,
-                              sweep_cluster_size(ms, 2 * (int)s.B, &spare));
+        int rc = launch_group(a, 0, (int)s.B, me, s, sweeps, st, ev, kStages);
         if (rc != FBW_B200_OK) return rc;
     }
     if (rc_forked != FBW_B200_OK) return rc_forked;
@@ -3104,9 +3197,7 @@ int fbw_b200_fbw_noalloc(const float* am, const int32_t* edges, const float* wei
     CUDA_OK(cudaMemsetAsync(sums, 0, sizeof(float) * (size_t)(sum.T * sum.B), st));
     i64 ms, me, md;
     plan_maxima(sum, ms, me, md);
-    int spare = sm_count() - 2 * (int)sum.B;
-    rc = launch_group(a, 0, (int)sum.B, ms, me, md, sum, st, nullptr, kDoAll,   // one stream, one chunk
-                      sweep_cluster_size(ms, 2 * (int)sum.B, &spare));
+    rc = launch_group(a, 0, (int)sum.B, me, sum, sweep_plan(sum), st, nullptr);  // one stream, one chunk
     if (rc != FBW_B200_OK) return rc;
     if (loss2) {
         k_loss<<<1, 1024, 0, st>>>(sums, sum.T, sum.B, loss2);
