@@ -887,8 +887,12 @@ struct RunArgs {
     float*       out;
     float*       sums;
     float*       loss2;
-    float *A, *Bt, *Gt, *Gf, *P;
-    float2* Gs;    // gathered scores as scaled numbers, frame-major (k_sweep_small); null: raw scores to Gf
+    float *A, *Bt, *Gt, *P;
+    // Gathered scores, frame-major: raw (Gf) or as scaled numbers for k_sweep_small (Gs, null otherwise), one array
+    // for both.  gf_scale: floats it has for a class and frame (2; 1 where it holds raw scores only).
+    float*  Gf;
+    float2* Gs;
+    int     gf_scale;
     const int *state_off, *edge_off, *slot_off, *nslot, *seq_T, *start_l, *end_l;
     const i64 *ta_off, *tg_off, *gf_off, *gu_off, *pu_off;
     const int *rowptr_f, *rowptr_b;
@@ -920,10 +924,18 @@ struct RunArgs {
     int fill_ctas;
     int fill_piece;   // floats per bulk store of the background (a multiple of 32, at most kFillFloats)
     int fill_offset;  // where the block of background starts in the sweep CTA's dynamic shared memory (bytes)
-    // 1: the frame-major score array Gf has been filled by the host (fbw_b200_run_with_host with scores in
-    // host memory); k_gather then only builds the tiled copy from it
-    int gathered_by_host;
+    // not null: the scores as the host has picked them out (fbw_b200_run_with_host with scores in host memory),
+    // frame-major like P; k_gather reads them in place of `am`
+    const float* picked;
 };
+
+// the raw scores of a sequence
+__device__ __forceinline__ float* raw_scores(const RunArgs& a, int b) { return a.Gf + a.gf_scale * a.gf_off[b]; }
+// The class posteriors of a sequence of Te frames, rows of Dp floats.  Without an array of their own they take
+// the second half of the sequence's scores, which the sweeps must have left.
+__device__ __forceinline__ float* posteriors(const RunArgs& a, int b, int Te, int Dp) {
+    return a.P ? a.P + a.gf_off[b] : a.Gf + 2 * a.gf_off[b] + (i64)Te * Dp;
+}
 
 // chunk in which the sweeps first need the scores of tile k of a sequence of Te frames: the forward
 // sweep reaches frame 32k at step 32k, the backward sweep reaches the tile's last frame at step
@@ -966,7 +978,7 @@ __global__ void __launch_bounds__(256) k_gather(RunArgs a) {
         const int d0 = c * kGatherSlots;
         const int nd = min(kGatherSlots, Db - d0);
         const int* __restrict__ emis = a.slot_emis + so + d0;
-        float* __restrict__ gf = a.Gf + a.gf_off[b];
+        float* __restrict__ gf = raw_scores(a, b);
         float2* __restrict__ gs = a.Gs ? a.Gs + a.gf_off[b] : nullptr;
         float* __restrict__ gt = a.Gt ? a.Gt + a.tg_off[b] + ((i64)k * Db + d0) * kTile : nullptr;
 
@@ -974,21 +986,21 @@ __global__ void __launch_bounds__(256) k_gather(RunArgs a) {
 #pragma unroll
         for (int j = 0; j < kGatherSlots / 32; j++) {
             int dd = lane + 32 * j;
-            em[j]  = dd < nd ? emis[dd] : 0;
+            em[j]  = dd < nd ? (a.picked ? dd : emis[dd]) : 0;
         }
         for (int f = warp; f < kTile; f += 8) {
             const int  t     = k * kTile + f;
             const bool valid = t < Te;
-            // (scores gathered by the host: the row of Gf itself, indexed by slot)
-            const float* row = a.gathered_by_host
-                                   ? gf + (i64)t * Dp + d0
+            // (scores picked out by the host: a row indexed by slot)
+            const float* row = a.picked
+                                   ? a.picked + a.gf_off[b] + (i64)t * Dp + d0
                                    : a.am + (a.fused ? ((i64)b * a.T + t) : ((i64)t * B + b)) * a.F;
             const float sgn = a.fused == 1 ? -1.f : 1.f;  // 2: batch-major input, sign kept
             float v[kGatherSlots / 32];
 #pragma unroll
             for (int j = 0; j < kGatherSlots / 32; j++) {
                 int dd = lane + 32 * j;
-                v[j]   = (valid && dd < nd) ? (a.gathered_by_host ? row[dd] : sgn * __ldg(row + em[j])) : CUDART_INF_F;
+                v[j]   = (valid && dd < nd) ? sgn * __ldg(row + em[j]) : CUDART_INF_F;
             }
 #pragma unroll
             for (int j = 0; j < kGatherSlots / 32; j++) {
@@ -996,13 +1008,13 @@ __global__ void __launch_bounds__(256) k_gather(RunArgs a) {
                 if (dd < nd) {
                     tile[f][dd] = v[j];
                     if (valid && gs) gs[(i64)t * Dp + d0 + dd] = to_scaled(v[j]);
-                    if (valid && !gs && !a.gathered_by_host) gf[(i64)t * Dp + d0 + dd] = v[j];
+                    if (valid && !gs) gf[(i64)t * Dp + d0 + dd] = v[j];
                 }
             }
             if (valid && c == nch - 1) {
                 for (int dd = Db + lane; dd < Dp; dd += 32) {
                     if (gs) gs[(i64)t * Dp + dd] = make_float2(0.f, CUDART_INF_F);
-                    else if (!a.gathered_by_host) gf[(i64)t * Dp + dd] = 0.f;
+                    else gf[(i64)t * Dp + dd] = 0.f;
                 }
             }
         }
@@ -1216,7 +1228,7 @@ __global__ void __launch_bounds__(1024) k_sweep(RunArgs a, int smax, int dpmax, 
         for (int k = 0; k < kRegEdges; k++) { rfrom[k] = 0; rslot[k] = 0; rw[k] = CUDART_INF_F; }
     }
 
-    const float* __restrict__ gf = a.Gf + a.gf_off[b];
+    const float* __restrict__ gf = raw_scores(a, b);
     float* __restrict__ dst = (fwd ? a.A : a.Bt) + a.ta_off[b];
     const int nvec = Dp >> 2;
     // frames whose scores are consumed: forward 0..Te-2, backward Te-1..1
@@ -1627,7 +1639,7 @@ __global__ void __launch_bounds__(32 * kPostWarps, 3) k_post(RunArgs a) {
         __syncthreads();
 
         // ---- posteriors, transposed: frame r of the tile gets its classes as one contiguous write ----
-        float* __restrict__ Pb = a.P + a.gf_off[p.b];
+        float* __restrict__ Pb = posteriors(a, p.b, p.Te, p.Dp);
         float (*st)[kTile + 1] = stage[warp];
         const float norm = fold ? 0.f : nm;  // (the differences are already taken)
         for (int d0 = warp * kTile; d0 < p.Db; d0 += W * kTile) {
@@ -1690,7 +1702,7 @@ __global__ void __launch_bounds__(256) k_expand(RunArgs a) {
         const int  Db = valid ? a.nslot[b] : 0;
         const int  Dp = (a.nslot[b] + 3) & ~3;
         const int* __restrict__ emis = a.slot_emis + so;
-        const float* __restrict__ Pr = a.P + a.gf_off[b] + (i64)t * Dp;
+        const float* __restrict__ Pr = posteriors(a, b, a.seq_T[b], Dp) + (i64)t * Dp;
         const i64 rbase = r * F;
         float* __restrict__ row = a.out + rbase;
         const int head = (int)min((i64)((4 - (rbase & 3)) & 3), F);
@@ -1810,7 +1822,7 @@ __global__ void __launch_bounds__(256) k_expand(RunArgs a) {
 // sector (slots are in ascending emission id, so they follow it) and writes the eight words.
 __device__ __forceinline__ void patch_row(const RunArgs& a, const PostUnit& p, int t, int lane) {
     const int* __restrict__ emis = a.slot_emis + p.so;
-    const float* __restrict__ Pr = a.P + a.gf_off[p.b] + (i64)t * p.Dp;
+    const float* __restrict__ Pr = posteriors(a, p.b, p.Te, p.Dp) + (i64)t * p.Dp;
     const i64 F     = a.F;
     // plain mode: background +inf, values are the negative log posteriors; fused mode: background 0,
     // values are -posterior, rows ordered (sequence, frame) (see k_expand)
@@ -1884,10 +1896,12 @@ __global__ void __launch_bounds__(1024) k_loss(const float* __restrict__ sums, i
 // host side
 // ---------------------------------------------------------------------------------------------
 struct RunLayout {
-    size_t A, Bt, Gt, Gf, Gs, P, carry, next_row, total;
+    size_t A, Bt, Gt, G, P, carry, next_row, total;
 };
 
-RunLayout run_layout(const fbw_b200_summary& s) {
+// own_post: the posteriors have an array of their own (the time chunks need it: a chunk's posteriors are written
+// while the sweeps still read scores)
+RunLayout run_layout(const fbw_b200_summary& s, bool own_post = true) {
     RunLayout L;
     size_t    off  = 0;
     auto      take = [&](size_t floats) {
@@ -1898,9 +1912,8 @@ RunLayout run_layout(const fbw_b200_summary& s) {
     L.A     = take((size_t)s.state_floats);
     L.Bt    = take((size_t)s.state_floats);
     L.Gt    = take((size_t)s.tiled_floats);
-    L.Gf    = take((size_t)s.frame_floats);
-    L.Gs    = take((size_t)s.frame_floats * 2);
-    L.P     = take((size_t)s.frame_floats);
+    L.G     = take((size_t)s.frame_floats * 2);
+    L.P     = own_post ? take((size_t)s.frame_floats) : 0;
     L.carry = take((size_t)(4 * s.S));
     L.next_row = take(2 * FBW_B200_GROUPS);  // a 64-bit row counter per group (background_rows)
     L.total = off;
@@ -1961,7 +1974,8 @@ void plan_args(RunArgs& a, const void* plan, const fbw_b200_summary& s) {
     a.fill_ctas = 0;
     a.fill_piece = kFillFloats;
     a.fill_offset = 0;
-    a.gathered_by_host = 0;
+    a.picked = nullptr;
+    a.gf_scale = 1;
 }
 
 // the arguments of one forward-backward call: plan arrays, run scratch, inputs and outputs
@@ -1974,9 +1988,10 @@ RunArgs fbw_args(const void* plan, const fbw_b200_summary& s, void* work, const 
     a.A  = at<float>(work, R.A);
     a.Bt = at<float>(work, R.Bt);
     a.Gt = at<float>(work, R.Gt);
-    a.Gf = at<float>(work, R.Gf);
-    a.Gs = at<float2>(work, R.Gs);
-    a.P  = at<float>(work, R.P);
+    a.Gf = at<float>(work, R.G);
+    a.Gs = at<float2>(work, R.G);
+    a.gf_scale = 2;
+    a.P  = R.P > 0 ? at<float>(work, R.P) : nullptr;
     a.carry = at<float>(work, R.carry);
     a.fused = fused;
     return a;
@@ -2808,7 +2823,7 @@ static int run_impl(const void* plan, const fbw_b200_summary* summary, const flo
         // Scores in host memory: reading the sectors the automata need over the bus takes 37 ms on the
         // triphone workload (32-byte read requests), and nothing else of the call can start before.  The
         // host threads pick them out of the tensor instead (a cache line per class, 13 ms) and one copy
-        // takes the 92 MB to the device; k_gather then only builds the tiled copy.
+        // takes the 92 MB to the device, where k_gather reads them.
         static int conf = -1;
         if (conf < 0) { const char* e = getenv("FBW_B200_HOST_GATHER"); conf = e ? atoi(e) : 1; }
         if (conf) {
@@ -2816,8 +2831,10 @@ static int run_impl(const void* plan, const fbw_b200_summary* summary, const flo
             host_rows.am = am;
             float* G = reinterpret_cast<float*>(static_cast<char*>(host_work) + H.G);
             if (!fbw_b200::host_gather(host_rows, G, host_nthreads)) return FBW_B200_BAD_ARGUMENT;
-            CUDA_OK(cudaMemcpyAsync(a.Gf, G, 4 * (size_t)s.frame_floats, cudaMemcpyHostToDevice, st));
-            a.gathered_by_host = 1;
+            // (to the posteriors' place on the device: a frame's row is read before its posteriors are written)
+            float* picked = at<float>(work, R.P);
+            CUDA_OK(cudaMemcpyAsync(picked, G, 4 * (size_t)s.frame_floats, cudaMemcpyHostToDevice, st));
+            a.picked = picked;
             host_scores = false;  // from here on the call is one whose scores are on the device
         }
     }
@@ -3185,7 +3202,7 @@ int fbw_b200_fbw_noalloc(const float* am, const int32_t* edges, const float* wei
     if (rc != FBW_B200_OK) return rc;
     // the size of the run scratch is known only now; the plan kernels have run on the array, the
     // caller's outputs are untouched
-    const RunLayout R = run_layout(sum);
+    const RunLayout R = run_layout(sum, false);
     if (plan_bytes + R.total > kNoAllocBytes) return FBW_B200_TOO_LARGE;
     void* work = static_cast<unsigned char*>(base) + plan_bytes;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);

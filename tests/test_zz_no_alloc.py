@@ -102,3 +102,19 @@ def test_noalloc_entry_rejects_what_does_not_fit(cuda):
     big = torch.zeros((1000, 16, 7000), dtype=torch.float32, device=cuda)
     rc, _, _, _ = _noalloc(lib, big, fsa, sl)
     assert rc == 5
+
+
+def test_noalloc_entry_takes_nine_lattices(cuda):
+    """Scratch per frame and class, edge and state: nine lattices over 5000 classes with few edges a class
+    (plan and run scratch about 46 MiB; with scaled and raw scores in arrays of their own it was 68)."""
+    import i6_native_ops_b200.fbw as m
+
+    lib = ctypes.CDLL(LIB)
+    lib.fbw_b200_fbw_noalloc.restype = ctypes.c_int
+    b = wl.make_batch("lattice", B=9, scale=0.2)
+    am = wl.make_scores(b, cuda)
+    fsa, sl = wl.to_torch(b, cuda)
+    rc, out, sums, _ = _noalloc(lib, am, fsa, sl)
+    assert rc == 0
+    ref_out, ref_sums = m.core.fbw(am, fsa[1], fsa[2], fsa[3], sl, int(fsa[0]), m.core.DebugOptions())
+    assert torch.equal(sums, ref_sums) and torch.equal(out, ref_out)
