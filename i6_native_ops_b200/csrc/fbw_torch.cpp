@@ -117,6 +117,10 @@ void write_output_dump(const torch::Tensor& out_dev, const torch::Tensor& seq_le
     }
 }
 
+// Calls of the op in this process, counted like the reference's static batch_idx (fbw_op.cu:246, 390); they
+// number the debug dumps.  fbw_loss counts whichever form of the op it takes.
+std::atomic<unsigned> call_counter{0};
+
 }  // namespace
 
 // The op.  Signature and meaning of the reference's fbw() (fbw_torch.cpp:15-29): am_scores (T,B,F)
@@ -138,9 +142,7 @@ std::vector<torch::Tensor> fbw(torch::Tensor& am_scores, torch::Tensor& edges,
     torch::Tensor sums = torch::empty({am_scores.size(0), am_scores.size(1)}, am_scores.options());
     Prepared p = prepare_impl(edges, weights, start_end_states, seq_lens, am_scores.size(0),
                               am_scores.size(2), (int64_t)num_states);
-    // dumps every `dump_every`-th call of the process, counted like the reference's static batch_idx
-    // (fbw_op.cu:246, 390)
-    static std::atomic<unsigned> call_counter{0};
+    // dumps every `dump_every`-th call of the process
     const unsigned call_idx = call_counter.fetch_add(1);
     const bool dump_now = debug_options.dump_every > 0 && call_idx % debug_options.dump_every == 0;
     torch::Tensor work;
@@ -251,7 +253,7 @@ static std::vector<torch::Tensor> run_fused_impl(const Prepared& p, const torch:
 // and neg/exp after it (i6_native_ops/fbw/__init__.py:41-44, 66); used by fbw_loss.
 std::vector<torch::Tensor> fbw_fused(torch::Tensor& log_probs, torch::Tensor& edges,
                                      torch::Tensor& weights, torch::Tensor& start_end_states,
-                                     torch::Tensor& seq_lens, int64_t num_states) {
+                                     torch::Tensor& seq_lens, int64_t num_states, bool counted) {
     check_input(log_probs, torch::kFloat32, "log_probs");
     TORCH_CHECK(log_probs.dim() == 3, "log_probs must have shape (B, T, F)");
     TORCH_CHECK(start_end_states.dim() == 2 && start_end_states.size(1) == log_probs.size(0),
@@ -264,6 +266,7 @@ std::vector<torch::Tensor> fbw_fused(torch::Tensor& log_probs, torch::Tensor& ed
     torch::Tensor grad = torch::empty_like(log_probs);
     torch::Tensor sums = torch::empty({T, B}, log_probs.options());
     Prepared p = prepare_impl(edges, weights, start_end_states, seq_lens, T, F, num_states);
+    if (counted) call_counter.fetch_add(1);
     return run_fused_impl(p, log_probs, grad, sums);
 }
 
@@ -412,7 +415,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("fbw_run_phases", &fbw_run_phases, "fbw_run with per-kernel device times");
     m.def("launch_count", []() { return fbw_b200_launch_count(); });
     m.def("fbw", &fbw, "Fast Baum-Welch CUDA routine (B200)");
-    m.def("fbw_fused", &fbw_fused, "fbw on (B,T,F) log_probs, returning the gradient directly");
+    m.def("fbw_fused", &fbw_fused,
+          "fbw on (B,T,F) log_probs, returning the gradient directly; `counted`: the call takes a number of the "
+          "debug dumps",
+          py::arg("log_probs"), py::arg("edges"), py::arg("weights"), py::arg("start_end_states"),
+          py::arg("seq_lens"), py::arg("num_states"), py::arg("counted") = false);
     m.def("fbw_host_scores", &fbw_host_scores,
           "fbw on scores in pinned host memory: only the scores the automata need cross the bus; "
           "`out`: optional pinned host tensor that receives the (T,B,F) result directly",

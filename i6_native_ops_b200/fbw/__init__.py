@@ -89,7 +89,7 @@ def fbw_loss(
         ``-posterior`` in ``log_probs.grad``.
     """
     if _read_in_place(log_probs):
-        return fbw_loss_fused(log_probs, fsa, seq_lens)
+        return FusedFastBaumWelchLoss.apply(log_probs.contiguous(), fsa, seq_lens, True)
     neg_log_probs = log_probs.neg().transpose(0, 1).contiguous()  # (T, B, F)
     return FastBaumWelchLoss.apply(neg_log_probs, fsa, seq_lens)  # the op says what it does not take
 
@@ -112,25 +112,26 @@ class FusedFastBaumWelchLoss(torch.autograd.Function):
     """``apply(log_probs (B,T,F), fsa, seq_lens) -> (T,B)`` per-frame sums, with the wrapper's
     elementwise passes done inside the kernels: the op reads ``log_probs`` in place (no negated,
     transposed copy) and writes ``d loss.sum() / d log_probs = -posterior`` directly in (B,T,F).
-    Like the reference's backward it does not scale by the incoming gradient."""
+    Like the reference's backward it does not scale by the incoming gradient.  ``counted``: the call takes a
+    number of the debug dumps (``DebugOptions.dump_every``), as calls of ``core.fbw`` do."""
 
     @staticmethod
-    def forward(ctx, log_probs, fsa, seq_lens):
+    def forward(ctx, log_probs, fsa, seq_lens, counted=False):
         num_states, edge_tensor, weight_tensor, start_end_states = fsa
         seq_lens = lengths_of(seq_lens, log_probs.shape[1], log_probs.shape[0])
         grad, loss = core.fbw_fused(log_probs, edge_tensor, weight_tensor, start_end_states,
-                                    seq_lens, int(num_states))
+                                    seq_lens, int(num_states), counted)
         ctx.save_for_backward(grad)
         return loss
 
     @staticmethod
     def backward(ctx, grad_loss):
-        return _gradient_of(ctx.saved_tensors[0]), None, None
+        return _gradient_of(ctx.saved_tensors[0]), None, None, None
 
 
 def fbw_loss_fused(log_probs, fsa, seq_lens):
     """What :func:`fbw_loss` does with float32 CUDA ``log_probs``, and nothing else: no negated or
-    transposed copy of the (B,T,F) tensor."""
+    transposed copy of the (B,T,F) tensor, and no number of the debug dumps."""
     return FusedFastBaumWelchLoss.apply(log_probs.contiguous(), fsa, seq_lens)
 
 

@@ -151,3 +151,24 @@ def test_dump_every_and_off_by_default(fbw_mod, cuda, tmp_path, monkeypatch):
     calls = sorted(int(os.path.basename(p).split(".")[2]) for p in files)
     assert len(calls) == 2 and all(c % 2 == 0 for c in calls)
     assert glob.glob(str(tmp_path / "alignment.dump.*")) == []
+
+
+def test_fbw_loss_counts_as_a_call(fbw_mod, cuda, tmp_path, monkeypatch):
+    """The dumps are numbered by the calls of the process (fbw_op.cu:246, 390); a training step through fbw_loss is
+    one of them."""
+    b = wl.make_batch("ctc_tiny")
+    am = wl.make_scores(b, cuda)
+    fsa, sl = wl.to_torch(b, cuda)
+    opts = fbw_mod.core.DebugOptions()
+    opts.dump_output, opts.dump_every = True, 1
+    monkeypatch.chdir(tmp_path)
+
+    def dumped():
+        before = set(glob.glob("target.dump.*.0"))
+        fbw_mod.core.fbw(am, fsa[1], fsa[2], fsa[3], sl, int(fsa[0]), opts)
+        (new,) = set(glob.glob("target.dump.*.0")) - before
+        return int(new.split(".")[2])
+
+    first = dumped()
+    fbw_mod.fbw_loss(am.neg().transpose(0, 1).contiguous(), fsa, sl)
+    assert dumped() == first + 2
