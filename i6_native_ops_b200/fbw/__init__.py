@@ -98,8 +98,9 @@ def _read_in_place(log_probs: torch.Tensor) -> bool:
     """Whether the op takes ``log_probs`` as they are.  The negated, transposed copy, and the passes that
     turn negative log posteriors (T,B,F) into the gradient (B,T,F), are nine sweeps over a tensor of up
     to gigabytes around an op that reads a small part of it (17 triphone sequences of 1499 frames and
-    12001 classes: 3.37 ms a training step, of which 2.3 ms)."""
-    return log_probs.dim() == 3 and log_probs.is_cuda and log_probs.dtype == torch.float32
+    12001 classes: 3.37 ms a training step, of which 2.3 ms).  A view that holds its values negated (torch's
+    negative bit) is copied."""
+    return log_probs.dim() == 3 and log_probs.is_cuda and log_probs.dtype == torch.float32 and not log_probs.is_neg()
 
 
 def _gradient_of(saved: torch.Tensor) -> torch.Tensor:

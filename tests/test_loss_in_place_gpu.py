@@ -8,7 +8,7 @@ from i6_native_ops_b200 import workloads as wl
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("layout", ["contiguous", "transposed", "offset", "strided"])
+@pytest.mark.parametrize("layout", ["contiguous", "transposed", "offset", "strided", "negated"])
 @pytest.mark.parametrize("cached", [False, True])
 def test_same_as_the_op_on_a_copy(cuda, layout, cached):
     import i6_native_ops_b200.fbw as m
@@ -24,6 +24,8 @@ def test_same_as_the_op_on_a_copy(cuda, layout, cached):
         x = lp
     elif layout == "offset":  # not aligned to 16 bytes
         x = torch.empty(B * T * F + 1, device=cuda)[1:].view(B, T, F).copy_(lp)
+    elif layout == "negated":  # a view whose sign is a bit of the tensor: the memory holds the negated values
+        x = torch._neg_view(lp.neg().contiguous())
     else:
         x = torch.empty(B, T, F, 2, device=cuda)[..., 0].copy_(lp)
     x = x.detach().requires_grad_(True)
