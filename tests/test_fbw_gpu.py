@@ -215,7 +215,8 @@ def test_full_size_triphone_properties(fbw_mod, ref_core, cuda):
                                      ("triphone", dict(B=20, T=600, F=4001, scale=0.4))])
 def test_fused_wrapper_matches_plain_wrapper(fbw_mod, cuda, name, kw):
     """fbw_loss_fused folds the wrapper's passes (i6_native_ops/fbw/__init__.py:41-44, 66) into
-    the kernels: same (T,B) loss, same gradient -posterior in (B,T,F)."""
+    the kernels: same (T,B) loss, same gradient -posterior in (B,T,F) as the op on a negated, transposed copy,
+    and as fbw_loss."""
     b = wl.make_batch(name, **kw)
     am = wl.make_scores(b, cuda)
     fsa, sl = wl.to_torch(b, cuda)
@@ -227,6 +228,12 @@ def test_fused_wrapper_matches_plain_wrapper(fbw_mod, cuda, name, kw):
     loss2.sum().backward()
     assert torch.equal(loss1, loss2)
     assert float((lp1.grad - lp2.grad).abs().max()) <= 1e-6
+    lp3 = lp1.detach().clone().requires_grad_(True)
+    loss3 = fbw_mod.FastBaumWelchLoss.apply(lp3.neg().transpose(0, 1).contiguous(), fsa, sl)
+    loss3.sum().backward()
+    assert torch.equal(loss3, loss2)
+    # exp of the same values by two implementations, each within 2 ulp of values at most 1
+    assert float((lp3.grad - lp2.grad).abs().max()) <= 4 * 2.0 ** -23
     t = torch.arange(b.T, device=cuda)[None, :, None]
     pad = (t >= sl[:, None, None]).expand_as(lp2.grad)
     assert bool((lp2.grad[pad] == 0).all())

@@ -98,6 +98,11 @@ def test_plan_cache_reuses_and_invalidates(mods, cuda):
     l2 = fbw.fbw_loss_cached(x2, fsa, sl, cache)
     l2.sum().backward()
     assert torch.equal(l1, l2) and torch.equal(x1.grad, x2.grad)
+    x0 = log_probs.clone().requires_grad_(True)  # the op itself, on a negated, transposed copy
+    l0 = fbw.FastBaumWelchLoss.apply(x0.neg().transpose(0, 1).contiguous(), fsa, sl)
+    l0.sum().backward()
+    assert torch.equal(l0, l2)
+    assert float((x0.grad - x2.grad).abs().max()) <= 4 * 2.0 ** -23  # exp by two implementations
     assert (cache.hits, cache.misses) == (0, 1)
     fbw.fbw_loss_cached(x2.detach(), fsa, sl, cache)
     assert (cache.hits, cache.misses) == (1, 1)
