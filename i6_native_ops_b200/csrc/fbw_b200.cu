@@ -12,7 +12,8 @@
 //               score arrays (frame-major for the sweeps, 32-frame tiles for the score pass).
 //   k_sweep,  : one persistent CTA, or cluster, per (sequence, direction); the automaton lives in shared
 //   k_sweep_small  memory and registers, frames are stepped with one barrier each, next frames' scores
-//               arrive by cp.async; state scores leave eight frames at a time (sweep_b200.inc).
+//               arrive by cp.async; state scores leave several frames at a time (sweep_scaled_b200.inc;
+//               k_sweep_cluster and, in sweep_cluster_b200.inc, k_sweepc on clusters).
 //   k_post    : per (sequence, 32 frames), lane = frame: edge scores, frame normalisers and class
 //               posteriors, none of which but the posteriors goes through memory.
 //   k_expand  : streams the (T,B,F) output: +inf rows with the few finite posteriors patched in.
@@ -73,7 +74,7 @@ struct PlanLayout {
     size_t qpos;                                                                 // int[E]
     size_t eiota, keyq, keyf, keyb, key32_out, qe, fe, be, me, slot_of_edge;     // [E]
     size_t key64, key64_out;                                                     // u64[E]
-    size_t head, hs, m_ptr;                                                      // int[E+1]
+    size_t head, hs;                                                             // int[E+1]
     size_t rowcnt_f, rowptr_f, rowcnt_b, rowptr_b;                               // int[S+1]
     size_t fwd_rec, bwd_rec;                                                     // uint2[E]
     size_t m_rec;                                                                // int4[E]
@@ -153,7 +154,6 @@ PlanLayout plan_layout(i64 B, i64 E, i64 S) {
     L.key64_out    = take(8 * nE);
     L.head         = take(4 * (nE + 1));
     L.hs           = take(4 * (nE + 1));
-    L.m_ptr        = take(4 * (nE + nB + 1));
     L.rowcnt_f     = take(4 * (nS + 1));
     L.rowptr_f     = take(4 * (nS + 1));
     L.rowcnt_b     = take(4 * (nS + 1));
@@ -446,19 +446,14 @@ __global__ void k_heads(const unsigned long long* __restrict__ key64s, i64 E, in
 __global__ void k_slots(const unsigned long long* __restrict__ key64s, const int* __restrict__ me,
                         const int* __restrict__ qe, const int* __restrict__ head,
                         const int* __restrict__ hs, i64 E, i64 F, int* slot_of_edge, int* slot_emis,
-                        int* m_ptr, int* qpos, const fbw_b200_summary* hdr) {
+                        int* qpos, const fbw_b200_summary* hdr) {
     if (hdr->error) return;
     i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < E) {
         qpos[qe[i]] = (int)i;  // position of an edge in the sequence-grouped ascending list
         int g = hs[i] + head[i] - 1;  // global slot of this edge
-        if (head[i]) {
-            slot_emis[g] = (int)(key64s[i] % (unsigned long long)F);
-            m_ptr[g]     = (int)i;
-        }
+        if (head[i]) slot_emis[g] = (int)(key64s[i] % (unsigned long long)F);
         slot_of_edge[me[i]] = g;
-    } else if (i == E) {
-        m_ptr[hs[E]] = (int)E;
     }
 }
 
@@ -502,10 +497,10 @@ __global__ void __launch_bounds__(1024) k_off2(const int* __restrict__ state_off
     __shared__ int smax[4];
     __shared__ int smin;
     __shared__ int gmax[3][FBW_B200_GROUPS];
-    // The eight offset arrays of up to kRowSeqs sequences are scanned by a warp each, side by side (32
-    // sequences: 13 -> 7 us for the kernel); larger batches by the block, one by one.
+    // The scans over up to kRowSeqs sequences (five, and two in rank order) take a warp each, side by side (32
+    // sequences: 13 -> 7 us for the kernel); larger batches the whole block, one by one.
     constexpr int kRowSeqs = 512;
-    __shared__ i64 rows[6][kRowSeqs];
+    __shared__ i64 rows[5][kRowSeqs];
     const bool in_rows = B <= kRowSeqs;
     const int  warp = threadIdx.x >> 5;
     if (threadIdx.x < 8) carry[threadIdx.x] = 0;
@@ -518,7 +513,7 @@ __global__ void __launch_bounds__(1024) k_off2(const int* __restrict__ state_off
     for (int base = 0; base < B; base += 1024) {
         int  b  = base + threadIdx.x;
         bool ok = b < B;
-        i64  v[6] = {0, 0, 0, 0, 0, 0};
+        i64  v[5] = {0, 0, 0, 0, 0};
         if (ok) {
             int Sb = state_off[b + 1] - state_off[b];
             int Eb = edge_off[b + 1] - edge_off[b];
@@ -539,8 +534,7 @@ __global__ void __launch_bounds__(1024) k_off2(const int* __restrict__ state_off
             v[1] = (i64)nt * Db * kTile;
             v[2] = (i64)Te * Dp;
             v[3] = Te;
-            v[4] = (i64)nt * Eb * kTile;
-            v[5] = Db;
+            v[4] = Db;
             cost[b] = (i64)Te * (Eb + 1);
             atomicMax(&smax[0], Sb);
             atomicMax(&smax[1], Eb);
@@ -548,20 +542,20 @@ __global__ void __launch_bounds__(1024) k_off2(const int* __restrict__ state_off
             atomicMax(&smax[3], Te);
             if (Te > 0) atomicMin(&smin, Te);
         }
-        i64* dst[6] = {ta_off, tg_off, gf_off, nullptr, nullptr, nullptr};
+        i64* dst[5] = {ta_off, tg_off, gf_off, nullptr, nullptr};
         if (in_rows) {
             if (ok) {
-                for (int k = 0; k < 6; k++) rows[k][b] = v[k];
+                for (int k = 0; k < 5; k++) rows[k][b] = v[k];
             }
             __syncthreads();
-            if (warp < 6) {
+            if (warp < 5) {
                 i64* to = warp == 0 ? ta_off : (warp == 1 ? tg_off : (warp == 2 ? gf_off : nullptr));
                 const i64 total = warp_offsets(rows[warp], B, to);
                 if ((threadIdx.x & 31) == 0) carry[warp] = total;
             }
             break;
         }
-        for (int k = 0; k < 6; k++) {
+        for (int k = 0; k < 5; k++) {
             i64 ex, agg;
             Scan(tmp).ExclusiveSum(v[k], ex, agg);
             if (ok && dst[k]) dst[k][b] = carry[k] + ex;
@@ -612,7 +606,7 @@ __global__ void __launch_bounds__(1024) k_off2(const int* __restrict__ state_off
             __syncthreads();
             if (warp < 2) {
                 const i64 total = warp_offsets(rows[warp], B, warp == 0 ? gu_off : pu_off);
-                if ((threadIdx.x & 31) == 0) carry[6 + warp] = total;
+                if ((threadIdx.x & 31) == 0) carry[5 + warp] = total;
             }
             __syncthreads();
             break;
@@ -620,9 +614,9 @@ __global__ void __launch_bounds__(1024) k_off2(const int* __restrict__ state_off
         for (int k = 0; k < 2; k++) {
             i64 ex, agg;
             Scan(tmp).ExclusiveSum(v[k], ex, agg);
-            if (ok) dst[k][r] = carry[6 + k] + ex;
+            if (ok) dst[k][r] = carry[5 + k] + ex;
             __syncthreads();
-            if (threadIdx.x == 0) carry[6 + k] += agg;
+            if (threadIdx.x == 0) carry[5 + k] += agg;
             __syncthreads();
         }
     }
@@ -630,17 +624,16 @@ __global__ void __launch_bounds__(1024) k_off2(const int* __restrict__ state_off
         ta_off[B] = carry[0];
         tg_off[B] = carry[1];
         gf_off[B] = carry[2];
-        gu_off[B] = carry[6];
-        pu_off[B] = carry[7];
-        hdr->score_floats = carry[4];
+        gu_off[B] = carry[5];
+        pu_off[B] = carry[6];
         hdr->T = T; hdr->B = B; hdr->F = F; hdr->E = E; hdr->S = S;
         hdr->state_floats = carry[0];
         hdr->tiled_floats = carry[1];
         hdr->frame_floats = carry[2];
         hdr->sum_len      = carry[3];
-        hdr->gather_units = carry[6];
-        hdr->post_units   = carry[7];
-        hdr->num_slots    = carry[5];
+        hdr->gather_units = carry[5];
+        hdr->post_units   = carry[6];
+        hdr->num_slots    = carry[4];
         hdr->max_states = smax[0];
         hdr->max_edges  = smax[1];
         hdr->max_slots  = smax[2];
@@ -697,7 +690,7 @@ struct FastSmem {
 template <int ITEMS>
 __device__ __forceinline__ void seqsort_lists(
     FastSmem& sm, const float* weights, i64 F, const int* qe, int e0, int Eb, int s0, int Sb, int so, int b,
-    int* rowptr_f, int* rowptr_b, uint2* fwd_rec, uint2* bwd_rec, int4* m_rec, int* m_ptr, int* slot_emis,
+    int* rowptr_f, int* rowptr_b, uint2* fwd_rec, uint2* bwd_rec, int4* m_rec, int* slot_emis,
     int* nslot, fbw_b200_summary* hdr) {
     const int tid = threadIdx.x;
     // (past-the-end keys are all ones: not below any key in the sorted bits, and behind their equals)
@@ -741,7 +734,6 @@ __device__ __forceinline__ void seqsort_lists(
             if (head[k]) {
                 slot++;
                 slot_emis[so + slot] = (int)(keys[k] >> kFastPosBits);
-                m_ptr[so + slot]     = e0 + j;
             }
             const int i = (int)(keys[k] & pos_mask);
             sm.slot[i] = (unsigned short)slot;
@@ -749,7 +741,6 @@ __device__ __forceinline__ void seqsort_lists(
         }
     }
     if (tid == 0) {
-        m_ptr[so + total] = e0 + Eb;
         nslot[b]          = total;
     }
     __syncthreads();
@@ -817,7 +808,7 @@ __global__ void __launch_bounds__(kFastThreads) k_seqsort(
     const int* __restrict__ edges, const float* __restrict__ weights, i64 E, i64 F,
     const int* __restrict__ qe, const int* __restrict__ edge_off, const int* __restrict__ state_off,
     const int* __restrict__ packed_of, int* rowptr_f, int* rowptr_b, uint2* fwd_rec, uint2* bwd_rec,
-    int4* m_rec, int* m_ptr, int* slot_emis, int* slot_off, int* nslot,
+    int4* m_rec, int* slot_emis, int* slot_off, int* nslot,
     fbw_b200_summary* hdr) {
     extern __shared__ __align__(16) unsigned char fast_raw[];
     FastSmem& sm = *reinterpret_cast<FastSmem*>(fast_raw);
@@ -844,10 +835,10 @@ __global__ void __launch_bounds__(kFastThreads) k_seqsort(
     __syncthreads();
     if (Eb <= kFastThreads * kFewItems) {
         seqsort_lists<kFewItems>(sm, weights, F, qe, e0, Eb, s0, Sb, so, b, rowptr_f, rowptr_b, fwd_rec, bwd_rec,
-                                 m_rec, m_ptr, slot_emis, nslot, hdr);
+                                 m_rec, slot_emis, nslot, hdr);
     } else {
         seqsort_lists<kFastItems>(sm, weights, F, qe, e0, Eb, s0, Sb, so, b, rowptr_f, rowptr_b, fwd_rec, bwd_rec,
-                                  m_rec, m_ptr, slot_emis, nslot, hdr);
+                                  m_rec, slot_emis, nslot, hdr);
     }
 }
 
@@ -898,7 +889,7 @@ struct RunArgs {
     const int *rowptr_f, *rowptr_b;
     const uint2 *fwd_rec, *bwd_rec;
     const int4* m_rec;  // {from | to << 16, position in ascending edge index, class slot, weight}, ordered by class
-    const int *m_ptr, *slot_emis, *order;
+    const int *slot_emis, *order;
     i64 T, B, F;
     int r0, r1;  // rank range (a group of sequences) this launch works on
     // Time chunks: the sweeps advance chunk_steps frames per chunk from both ends of a sequence; a
@@ -1964,7 +1955,6 @@ void plan_args(RunArgs& a, const void* plan, const fbw_b200_summary& s) {
     a.fwd_rec  = at<uint2>(plan, L.fwd_rec);
     a.bwd_rec  = at<uint2>(plan, L.bwd_rec);
     a.m_rec    = at<int4>(plan, L.m_rec);
-    a.m_ptr     = at<int>(plan, L.m_ptr);
     a.slot_emis = at<int>(plan, L.slot_emis);
     a.order     = at<int>(plan, L.order);
     a.T = s.T; a.B = s.B; a.F = s.F;
@@ -2568,7 +2558,6 @@ static int prepare_impl(const int32_t* edges, const float* weights, const int32_
         CUDA_OK(cudaMemsetAsync(at<int>(plan, L.rowcnt_f), 0, 4 * (size_t)(S + 1), st));
         CUDA_OK(cudaMemsetAsync(at<int>(plan, L.rowcnt_b), 0, 4 * (size_t)(S + 1), st));
         CUDA_OK(cudaMemsetAsync(at<int>(plan, L.hs), 0, 4 * (size_t)(E + 1), st));
-        CUDA_OK(cudaMemsetAsync(at<int>(plan, L.m_ptr), 0, 4 * (size_t)(E + B + 1), st));
     }
 
     const int TB = 256;
@@ -2623,7 +2612,7 @@ static int prepare_impl(const int32_t* edges, const float* weights, const int32_
             edges, weights, E, F, at<int>(plan, L.qe), at<int>(plan, L.edge_off),
             at<int>(plan, L.state_off), at<int>(plan, L.packed_of), at<int>(plan, L.rowptr_f),
             at<int>(plan, L.rowptr_b), at<uint2>(plan, L.fwd_rec), at<uint2>(plan, L.bwd_rec),
-            at<int4>(plan, L.m_rec), at<int>(plan, L.m_ptr), at<int>(plan, L.slot_emis), at<int>(plan, L.slot_off),
+            at<int4>(plan, L.m_rec), at<int>(plan, L.slot_emis), at<int>(plan, L.slot_off),
             at<int>(plan, L.nslot), hdr);
     } else if (E > 0) {
         k_edgekeys<<<blocks(E), TB, 0, st>>>(edges, E, F, at<int>(plan, L.packed_of),
@@ -2661,7 +2650,7 @@ static int prepare_impl(const int32_t* edges, const float* weights, const int32_
                                               at<int>(plan, L.me), at<int>(plan, L.qe),
                                               at<int>(plan, L.head), at<int>(plan, L.hs), E, F,
                                               at<int>(plan, L.slot_of_edge),
-                                              at<int>(plan, L.slot_emis), at<int>(plan, L.m_ptr),
+                                              at<int>(plan, L.slot_emis),
                                               at<int>(plan, L.qpos), hdr);
     } else {
         CUDA_OK(cudaMemsetAsync(at<int>(plan, L.rowptr_f), 0, 4 * (size_t)(S + 1), st));
