@@ -25,8 +25,8 @@
 //
 // Arithmetic.  Scores grow with t (~2e4 at T=1500, one ulp = 2e-3), and a sum of two of them rounded to
 // that grid, as the reference forms it, shows in the posteriors:
-//   * the sweeps' log-sums are formed in scaled numbers (scaled.h): a step rounds to about 2^-23 of the frame's
-//     own score, or of the sum where that is below one, whatever the accumulated score.  A stored state score is
+//   * the sweeps' log-sums are formed in scaled numbers (scaled.h): a step rounds to about 2^-23 of one, or of the
+//     sum where that is smaller, whatever the accumulated score.  A stored state score is
 //     the natural negative log, rounded once; it is closer to the exact value than the reference's.
 //     (Sweeps of automata with several states per thread add logarithms, as the reference does.)
 //   * prob_add is fbw_op.cu:39-48 in meaning: min(a,b) - log1p(exp(-|a-b|)), +inf where both are +inf,
@@ -196,7 +196,8 @@ __device__ __forceinline__ float ex2_approx(float x) {
 // Log-semiring sum of two negative-log values: min(a,b) - log1p(exp(-|a-b|)), the reference's prob_add
 // (i6_native_ops/fbw/fbw_op.cu:39-48).  log1p(e) on [0,1] is e times a polynomial of degree 8, fitted
 // here by linear programming (largest absolute error of e * q(e) 4.6e-10 before rounding, 1.3e-7 with
-// fp32 coefficients and steps); the last step is one fused multiply-add, so the sum is rounded once, to
+// fp32 coefficients and steps, 2.4e-7 with the hardware exponential's own error, relative to e where e is
+// small); the last step is one fused multiply-add, so the sum is rounded once, to
 // the grid of the scores, as in the reference.  Scores are sums over frames (magnitudes of 1e2..1e4, one
 // ulp 8e-6..1e-3), so the error of the logarithm disappears in that rounding: results are the
 // reference's but for a last-place step once in several hundred sums.
@@ -2087,7 +2088,8 @@ int sweep_cluster_size(i64 ms, int items, int* spare) {
     }
     if (forced == 1 || forced == 2 || forced == 4 || forced == 8) return forced;
     if (ms <= 1024 || items <= 0) return 1;
-    // (8 lattice sequences, ms a training step: clusters of two 5.7, of four 4.2, of eight 3.4)
+    // (8 lattice sequences, ms a training step: one CTA 8.6, clusters of two 6.3, of four 5.0, of eight 3.2; 128 lattice
+    // sequences, ms a call: 21.6, 19.2, 22.5, 29.6, by this rule 14.6)
     for (int cs = ms > 2048 ? 8 : 4; cs > 1; cs >>= 1) {
         const int extra = (cs - 1) * items;
         if (extra <= *spare) {
@@ -3129,7 +3131,7 @@ int64_t fbw_b200_launch_count(void) { return (int64_t)g_launches.load(); }
 // them the plan and the run scratch live in one fixed array inside the library image.  Every GPU
 // that loads the library carries the array until the process exits, so it is kept modest: 64 MiB,
 // enough for the small and medium workloads (a 32-sequence, 500-frame monophone batch needs about
-// 45 MiB), not for the 1 GB of scratch of the large ones.
+// 30 MiB), not for the 0.6 GB of scratch of the large ones.
 constexpr size_t kNoAllocBytes = (size_t)64 << 20;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 

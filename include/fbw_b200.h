@@ -261,7 +261,7 @@ int64_t fbw_b200_launch_count(void);
  * receives input and output buffers from its host and has no allocator to ask for scratch.  The plan
  * and the run scratch live in a fixed array inside the library (fbw_b200_noalloc_capacity() bytes,
  * 64 MiB, held by every GPU that loads the library until the process exits).  Same inputs and
- * outputs as fbw_b200_prepare + fbw_b200_run; loss2 may be NULL.  It has no counterpart in the
+ * outputs, bit for bit, as fbw_b200_prepare + fbw_b200_run; loss2 may be NULL.  It has no counterpart in the
  * reference, whose launcher allocates and frees per call (fbw_op.cu:283-286, 384-389).
  *  - Returns FBW_B200_TOO_LARGE when plan + scratch exceed the capacity, or when T*B*F >= 1e8 (a fixed
  *    cap: this entry runs its stages one after another on the caller's stream, which suits small and
