@@ -13,7 +13,8 @@
 //   k_sweep,  : one persistent CTA, or cluster, per (sequence, direction); the automaton lives in shared
 //   k_sweep_small  memory and registers, frames are stepped with one barrier each, next frames' scores
 //               arrive by cp.async; state scores leave several frames at a time (sweep_scaled_b200.inc;
-//               k_sweep_cluster and, in sweep_cluster_b200.inc, k_sweepc on clusters).
+//               k_sweep_cluster and, in sweep_cluster_b200.inc, k_sweepc on clusters; k_sweep_block for the
+//               smallest automata, sweep_block_b200.inc).
 //   k_post    : per (sequence, 32 frames), lane = frame: edge scores, frame normalisers and class
 //               posteriors, none of which but the posteriors goes through memory.
 //   k_expand  : streams the (T,B,F) output: +inf rows with the few finite posteriors patched in.
@@ -685,6 +686,7 @@ struct FastSmem {
     int      emis[kFastCap];
     unsigned last[kFastThreads];   // each thread's last sorted key (for the head test)
     int      deg_max;
+    int      groups[2];            // of three edges, by target state and by source state
 };
 
 // the three sorted lists of a sequence (see k_seqsort)
@@ -772,7 +774,7 @@ __device__ __forceinline__ void seqsort_lists(
         __syncthreads();
         // row pointers: first position whose state is >= s; the entry after the last state is the
         // first entry of the next sequence (both write the same value)
-        int dmax = 0;
+        int dmax = 0, groups = 0;
         for (int s = tid; s <= Sb; s += kFastThreads) {
             const unsigned want = (unsigned)s << kFastPosBits;
             int lo = 0, hi = Eb;
@@ -789,13 +791,18 @@ __device__ __forceinline__ void seqsort_lists(
                     if (sm.sorted[mid] < nxt) l2 = mid + 1; else h2 = mid;
                 }
                 dmax = max(dmax, l2 - lo);
+                groups += max(1, (l2 - lo + 2) / 3);
             }
         }
         if (dmax > 0) atomicMax(&sm.deg_max, dmax);
+        if (groups > 0) atomicAdd(&sm.groups[dir], groups);
         __syncthreads();
     }
     if (tid == 0 && sm.deg_max > 0) {
         atomicMax((unsigned long long*)&hdr->max_degree, (unsigned long long)sm.deg_max);
+    }
+    if (tid == 0) {  // (see edge_groups)
+        atomicMax((unsigned long long*)&hdr->reserved[0], (unsigned long long)max(sm.groups[0], sm.groups[1]));
     }
 }
 
@@ -826,7 +833,7 @@ __global__ void __launch_bounds__(kFastThreads) k_seqsort(
         }
         return;
     }
-    if (tid == 0) sm.deg_max = 0;
+    if (tid == 0) sm.deg_max = sm.groups[0] = sm.groups[1] = 0;
     for (int i = tid; i < Eb; i += kFastThreads) {
         const int e = qe[e0 + i];
         sm.from[i] = (unsigned short)(packed_of[edges[e]] - s0);
@@ -949,7 +956,7 @@ __device__ __forceinline__ bool in_chunks(int c, const RunArgs& a) { return c >=
 // Gather am_scores[t,b,emission] for the distinct emissions ("slots", ascending emission id) of
 // each sequence.  Work item = (sequence, 32-frame tile, 256 slots).  Two copies are written:
 //   Gf  frame-major  [t][slot]           (rows padded to 4 floats)  -- read by the sweeps, or instead
-//   Gs  the same as scaled numbers                                  -- read by k_sweep_small
+//   Gs  the same as scaled numbers                                  -- read by k_sweep_small and k_sweep_block
 //   Gt  tiled        [t/32][slot][t%32]                              -- read by k_post, lane = frame
 __global__ void __launch_bounds__(256) k_gather(RunArgs a) {
     __shared__ float tile[kTile][kGatherSlots + 1];
@@ -2073,6 +2080,7 @@ int launch_sweep(const RunArgs& a, int grid, int nt, size_t smem, int smax, int 
 
 #include "sweep_cluster_b200.inc"
 #include "sweep_scaled_b200.inc"
+#include "sweep_block_b200.inc"
 
 // CTAs per cluster for the sweeps of `items` (sequence, direction) pairs of automata of at most ms
 // states, when `spare` SMs would otherwise stay idle during the call's sweeps.  A cluster spreads the
@@ -2276,6 +2284,7 @@ struct SweepPlan {
     bool two_step;  // and whether it writes the output in two steps (given a destination that allows it)
     bool clustered;
     bool scaled[FBW_B200_GROUPS];
+    bool block[FBW_B200_GROUPS];  // k_sweep_block
     int  cs[FBW_B200_GROUPS];
 };
 int base_rank(const fbw_b200_summary& s, int q) { return (int)(((i64)q * s.B) / FBW_B200_GROUPS); }
@@ -2328,11 +2337,15 @@ SweepPlan sweep_plan(const fbw_b200_summary& s) {
         const int items = 2 * (base_rank(s, q0 + per) - base_rank(s, q0));
         // (the background of an output in two steps is written by the sweeps of one CTA)
         const int cs = p.two_step ? 1 : sweep_cluster_size(gs, items, &spare);
-        const bool scaled = scaled_shape(gs, ge, gd, s.max_degree, cs).found;
+        // (where the background is written and more sweep CTAs wait than fit two to an SM, the smaller ones of
+        // k_sweep_small hold it up less: 256 BPE-CTC sequences 983 against 995 us)
+        const bool block  = cs == 1 && block_shape(s, gs, gd).found && !(p.two_step && s.B > (i64)sm_count());
+        const bool scaled = block || scaled_shape(gs, ge, gd, s.max_degree, cs).found;
         p.clustered = p.clustered || cs > 1;
         for (int q = q0; q < q0 + per; q++) {
             p.cs[q]     = cs;
             p.scaled[q] = scaled;
+            p.block[q]  = block;
         }
     }
     return p;
@@ -2341,7 +2354,7 @@ SweepPlan sweep_plan(const fbw_b200_summary& s) {
 // The ranks [r0, r1) as runs of base groups that one sweep launch can serve
 struct SweepRun {
     int  r0, r1, cs;
-    bool scaled;
+    bool scaled, block;
     i64  ms, me, md;
 };
 int sweep_runs(const fbw_b200_summary& s, const SweepPlan& p, int r0, int r1, SweepRun* runs) {
@@ -2353,16 +2366,18 @@ int sweep_runs(const fbw_b200_summary& s, const SweepPlan& p, int r0, int r1, Sw
         if (r.r1 <= r.r0) continue;
         r.cs = p.cs[q];
         r.scaled = p.scaled[q];
+        r.block  = p.block[q];
         r.ms = s.group_max_states[q];
         r.me = s.group_max_edges[q];
         r.md = s.group_max_slots[q];
-        if (n > 0 && runs[n - 1].cs == r.cs && runs[n - 1].scaled == r.scaled) {
+        if (n > 0 && runs[n - 1].cs == r.cs && runs[n - 1].scaled == r.scaled && runs[n - 1].block == r.block) {
             SweepRun u = runs[n - 1];
             u.r1 = r.r1;
             u.ms = r.ms > u.ms ? r.ms : u.ms;
             u.me = r.me > u.me ? r.me : u.me;
             u.md = r.md > u.md ? r.md : u.md;
-            if (!u.scaled || scaled_shape(u.ms, u.me, u.md, s.max_degree, u.cs).found) {
+            if (u.block ? block_shape(s, u.ms, u.md).found
+                        : !u.scaled || scaled_shape(u.ms, u.me, u.md, s.max_degree, u.cs).found) {
                 runs[n - 1] = u;
                 continue;
             }
@@ -2392,7 +2407,17 @@ int launch_sweeps(RunArgs a, const SweepRun& r, const fbw_b200_summary& s, cudaS
     const i64 ms = r.ms, me = r.me, md = r.md;
     a.r0 = r.r0;
     a.r1 = r.r1;
-    if (r.scaled) {
+    if (r.block) {
+        const BlockShape bs = block_shape(s, ms, md);
+        size_t smem = bs.smem;
+        if (a.next_row != nullptr) {  // (as below)
+            a.fill_offset = (int)((bs.smem + 127) & ~(size_t)127);
+            smem = (size_t)a.fill_offset + sizeof(float) * (size_t)a.fill_piece;
+        }
+        const int rc = launch_block(a, bs, 2 * nb + (a.next_row != nullptr ? a.fill_ctas : 0),
+                                    bs.nt + (a.next_row != nullptr ? 32 : 0), smem, st);
+        if (rc != FBW_B200_OK) return rc;
+    } else if (r.scaled) {
         const ScaledShape sc = scaled_shape(ms, me, md, s.max_degree, cs);
         int rc;
         if (cs > 1) {

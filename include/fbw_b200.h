@@ -79,7 +79,7 @@ typedef struct fbw_b200_summary {
     int64_t max_degree;   /* largest in-degree or out-degree of a state                           */
     int64_t score_floats; /* 0 (there is no per-frame edge-score array any more)                   */
     int64_t min_len;      /* shortest valid sequence length (0 if none)                           */
-    int64_t reserved[1];
+    int64_t reserved[1];  /* about the edges of the states, for the choice of sweep                   */
 } fbw_b200_summary;
 
 /* Bytes of plan scratch for B sequences, E edges, S states. */
