@@ -307,11 +307,10 @@ __global__ void k_mark(const int* __restrict__ edges, const int* __restrict__ st
     }
 }
 
-// single block: exclusive scans of the per-sequence state and edge counts; effective lengths
-__global__ void __launch_bounds__(1024) k_off1(const int* __restrict__ scount,
-                                              const int* __restrict__ ecount,
-                                              const int* __restrict__ seq_lens, int B, i64 T,
-                                              int* state_off, int* edge_off, int* seq_T) {
+// one block of 1024: exclusive scans of the per-sequence state and edge counts; effective lengths
+__device__ __forceinline__ void sequence_offsets(const int* __restrict__ scount, const int* __restrict__ ecount,
+                                                 const int* __restrict__ seq_lens, int B, i64 T, int* state_off,
+                                                 int* edge_off, int* seq_T) {
     typedef cub::BlockScan<int, 1024> Scan;
     __shared__ typename Scan::TempStorage tmp;
     __shared__ int carry[2];
@@ -342,40 +341,38 @@ __global__ void __launch_bounds__(1024) k_off1(const int* __restrict__ scount,
         edge_off[B]  = carry[1];
     }
 }
+__global__ void __launch_bounds__(1024) k_off1(const int* __restrict__ scount,
+                                              const int* __restrict__ ecount,
+                                              const int* __restrict__ seq_lens, int B, i64 T,
+                                              int* state_off, int* edge_off, int* seq_T) {
+    sequence_offsets(scount, ecount, seq_lens, B, T, state_off, edge_off, seq_T);
+}
 
 __global__ void k_statekeys(const int* __restrict__ state_key, i64 S, int B, unsigned* skey,
-                            int* siota, int* unordered) {
+                            int* siota) {
     i64 s = (i64)blockIdx.x * blockDim.x + threadIdx.x;
     if (s < S) {
         int k    = state_key[s];
         skey[s]  = k < 0 ? (unsigned)B : (unsigned)k;
         siota[s] = (int)s;
-        // state ids usually run sequence after sequence (unused ids last); then ordering the states
-        // by owning sequence is the identity
-        if (s > 0) {
-            const int kp = state_key[s - 1];
-            if ((k < 0 ? B : k) < (kp < 0 ? B : kp)) unordered[1] = 1;
-        }
     }
 }
 
 // Stable grouping of n items by key (a counting sort with known group offsets `off`), one CTA:
-// perm[position] = item, inv[item] = position (inv may be null).  If the keys are already in
-// non-decreasing order (*unordered == 0) the grouping is the identity and is written as such; that
-// is the common case, and it replaces a device-wide radix sort (three kernels and two memsets) by
-// one short kernel.  Otherwise the items are taken 1024 at a time, the warps of a chunk one after
+// perm[position] = item, inv[item] = position (either may be null).  If the keys are already in
+// non-decreasing order (`ordered`) the grouping is the identity and is written as such; that
+// is the common case, and it replaces a device-wide radix sort (three kernels and two memsets).
+// Otherwise the items are taken 1024 at a time, the warps of a chunk one after
 // another, so that equal keys keep their order.
 constexpr int kGroupKeys = 8192;
-__global__ void __launch_bounds__(1024) k_group(const unsigned* __restrict__ keys, i64 n, int nkeys,
-                                                const int* __restrict__ off,
-                                                const int* __restrict__ unordered, int* perm, int* inv,
-                                                const fbw_b200_summary* hdr) {
-    __shared__ int cnt[kGroupKeys + 1];
-    if (hdr->error) return;
+template <typename Key>
+__device__ __forceinline__ void group_items(Key key, i64 n, int nkeys, const int* off, bool ordered, int* cnt, int* perm,
+                                            int* inv) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (*unordered == 0) {
+    if (ordered) {
+#pragma unroll 4
         for (i64 i = tid; i < n; i += 1024) {
-            perm[i] = (int)i;
+            if (perm) perm[i] = (int)i;
             if (inv) inv[i] = (int)i;
         }
         return;
@@ -385,7 +382,7 @@ __global__ void __launch_bounds__(1024) k_group(const unsigned* __restrict__ key
     for (i64 base = 0; base < n; base += 1024) {
         const i64  i  = base + tid;
         const bool in = i < n;
-        const unsigned k = in ? keys[i] : 0xffffffffu;  // items past the end form a group of their own
+        const unsigned k = in ? key(i) : 0xffffffffu;  // items past the end form a group of their own
         const unsigned peers = __match_any_sync(0xffffffffu, k);
         const int rank   = __popc(peers & ((1u << lane) - 1u));
         const int leader = __ffs(peers) - 1;
@@ -400,10 +397,37 @@ __global__ void __launch_bounds__(1024) k_group(const unsigned* __restrict__ key
         first = __shfl_sync(0xffffffffu, first, leader);
         if (in) {
             const int pos = off[k] + first + rank;
-            perm[pos] = (int)i;
+            if (perm) perm[pos] = (int)i;
             if (inv) inv[i] = pos;
         }
     }
+    __syncthreads();
+}
+
+// Batches of fewer than kGroupKeys sequences whose sequences are sorted by a CTA each: offsets and lengths of the
+// sequences, states grouped by owning sequence (stable: ascending state id inside a sequence; the keys 0..B, B = a
+// state that no sequence uses), edges grouped by sequence.  One CTA, in place of four launches of 1 to 5 us that
+// waited for one another.
+__global__ void __launch_bounds__(1024) k_order(const int* __restrict__ state_key, i64 S, const int* __restrict__ edge_seq,
+                                               i64 E, const int* __restrict__ scount, const int* __restrict__ ecount,
+                                               const int* __restrict__ seq_lens, int B, i64 T, int* state_off,
+                                               int* edge_off, int* seq_T, const int* __restrict__ unordered,
+                                               int* packed_of, int* qe, const fbw_b200_summary* hdr) {
+    __shared__ int cnt[kGroupKeys + 1];
+    sequence_offsets(scount, ecount, seq_lens, B, T, state_off, edge_off, seq_T);
+    if (hdr->error) return;
+    // state ids usually run sequence after sequence (unused ids last); then ordering them is the identity
+    auto key = [&](i64 s) {
+        const int k = state_key[s];
+        return k < 0 ? (unsigned)B : (unsigned)k;
+    };
+    bool descent = false;
+#pragma unroll 4
+    for (i64 s = threadIdx.x + 1; s < S; s += 1024) descent |= key(s) < key(s - 1);
+    const bool ordered = !__syncthreads_or(descent);  // (also: the offsets are there)
+    group_items(key, S, B + 1, state_off, ordered, cnt, nullptr, packed_of);
+    // the sequence ids of the edges are the keys (validated by k_mark, which flags the plan otherwise)
+    group_items([&](i64 e) { return (unsigned)edge_seq[e]; }, E, B, edge_off, *unordered == 0, cnt, qe, nullptr);
 }
 
 __global__ void k_packed(const int* __restrict__ sorted_state, i64 S, int* packed_of) {
@@ -2592,26 +2616,25 @@ static int prepare_impl(const int32_t* edges, const float* weights, const int32_
     void*  ctemp = at<char>(plan, L.cub_temp);
     size_t cbytes = L.cub_temp_bytes;
 
-    COUNT_LAUNCH(fast ? 7 : (E > 0 ? 9 : 5));  // k_mark, k_off1, k_statekeys, k_packed, k_off2 + edge kernels
     int* unordered = at<int>(plan, L.unordered);
-    // grouping by sequence with one CTA instead of a device-wide sort (see k_group)
+    // grouping by sequence with one CTA instead of device-wide sorts (see k_order)
     const bool group1 = fast && B < kGroupKeys;
+    COUNT_LAUNCH(group1 ? 4 : (fast ? 7 : (E > 0 ? 9 : 5)));  // k_mark, k_order or k_off1, k_statekeys, k_packed; k_off2; edge kernels
     k_mark<<<blocks(E + B), TB, 0, st>>>(edges, start_end, E, B, S, F, at<int>(plan, L.state_key),
                                          at<int>(plan, L.scount), at<int>(plan, L.ecount), unordered,
                                          hdr);
-    k_off1<<<1, 1024, 0, st>>>(at<int>(plan, L.scount), at<int>(plan, L.ecount), seq_lens, (int)B,
-                               T, at<int>(plan, L.state_off), at<int>(plan, L.edge_off),
-                               at<int>(plan, L.seq_T));
-    // states ordered by owning sequence (stable: ascending state id inside a sequence)
-    k_statekeys<<<blocks(S), TB, 0, st>>>(at<int>(plan, L.state_key), S, (int)B,
-                                          at<unsigned>(plan, L.skey), at<int>(plan, L.siota),
-                                          unordered);
     if (group1) {
-        // keys 0..B (B = state id not used by any sequence), group offsets = state_off[0..B]
-        k_group<<<1, 1024, 0, st>>>(at<unsigned>(plan, L.skey), S, (int)B + 1,
-                                    at<int>(plan, L.state_off), unordered + 1,
-                                    at<int>(plan, L.sorted_state), at<int>(plan, L.packed_of), hdr);
+        k_order<<<1, 1024, 0, st>>>(at<int>(plan, L.state_key), S, edges + 3 * E, E, at<int>(plan, L.scount),
+                                    at<int>(plan, L.ecount), seq_lens, (int)B, T, at<int>(plan, L.state_off),
+                                    at<int>(plan, L.edge_off), at<int>(plan, L.seq_T), unordered,
+                                    at<int>(plan, L.packed_of), at<int>(plan, L.qe), hdr);
     } else {
+        k_off1<<<1, 1024, 0, st>>>(at<int>(plan, L.scount), at<int>(plan, L.ecount), seq_lens, (int)B,
+                                   T, at<int>(plan, L.state_off), at<int>(plan, L.edge_off),
+                                   at<int>(plan, L.seq_T));
+        // states ordered by owning sequence (stable: ascending state id inside a sequence)
+        k_statekeys<<<blocks(S), TB, 0, st>>>(at<int>(plan, L.state_key), S, (int)B,
+                                              at<unsigned>(plan, L.skey), at<int>(plan, L.siota));
         CUDA_OK(cub::DeviceRadixSort::SortPairs(ctemp, cbytes, at<unsigned>(plan, L.skey),
                                                 at<unsigned>(plan, L.skey_out),
                                                 at<int>(plan, L.siota), at<int>(plan, L.sorted_state),
@@ -2619,13 +2642,7 @@ static int prepare_impl(const int32_t* edges, const float* weights, const int32_
         k_packed<<<blocks(S), TB, 0, st>>>(at<int>(plan, L.sorted_state), S, at<int>(plan, L.packed_of));
     }
     if (fast) {
-        if (group1) {
-            // the sequence ids of the edges are the keys (validated by k_mark, which flags the plan
-            // otherwise), group offsets = edge_off
-            k_group<<<1, 1024, 0, st>>>(reinterpret_cast<const unsigned*>(edges + 3 * E), E, (int)B,
-                                        at<int>(plan, L.edge_off), unordered, at<int>(plan, L.qe),
-                                        nullptr, hdr);
-        } else {
+        if (!group1) {
             k_seqkeys<<<blocks(E), TB, 0, st>>>(edges, E, at<unsigned>(plan, L.keyq),
                                                 at<int>(plan, L.eiota), hdr);
             CUDA_OK(cub::DeviceRadixSort::SortPairs(ctemp, cbytes, at<unsigned>(plan, L.keyq),
