@@ -80,6 +80,7 @@ struct PlanLayout {
     size_t fwd_rec, bwd_rec;                                                     // uint2[E]
     size_t m_rec;                                                                // int4[E]
     size_t slot_emis;                                                            // int[E]
+    size_t hops_f, hops_b;                                                       // int[S], where skey and siota were
     size_t cub_temp, cub_temp_bytes;
     size_t total;
 };
@@ -123,6 +124,8 @@ PlanLayout plan_layout(i64 B, i64 E, i64 S) {
     L.siota        = take(4 * nS);
     L.sorted_state = take(4 * nS);
     L.packed_of    = take(4 * nS);
+    L.hops_f       = L.skey;   // the states are sorted by then
+    L.hops_b       = L.siota;
     L.scount       = take(4 * (nB + 1));
     L.ecount       = take(4 * (nB + 1));
     L.unordered    = take(16);  // cleared together with the two count arrays before it
@@ -500,6 +503,104 @@ __device__ __forceinline__ i64 warp_offsets(const i64* row, int n, i64* dst) {
         carry += __shfl_sync(0xffffffffu, sum, 31);
     }
     return carry;
+}
+
+// Notes about the edges of a batch for the choice of sweep (fbw_b200_summary.reserved; general path): the furthest that
+// an edge leads on, 65535 if one leads back (bits 32 to 47), and the most groups of four that the edges of a
+// sequence's states take, by target or by source state (bits 48 to 63).
+__device__ __forceinline__ void note_edges(fbw_b200_summary* hdr, int reach, int groups) {
+    unsigned* word = reinterpret_cast<unsigned*>(&hdr->reserved[0]) + 1;
+    unsigned old = *(volatile unsigned*)word;
+    for (;;) {
+        const unsigned now = max(old & 0xffffu, (unsigned)min(reach, 0xffff)) | max(old >> 16, (unsigned)min(groups, 0xffff)) << 16;
+        const unsigned was = now == old ? old : atomicCAS(word, old, now);
+        if (was == old) break;
+        old = was;
+    }
+}
+// How many frames a state is from the sequence's start (forward) or from its end (backward) at least, for left-to-right
+// automata: the fewest steps if from every state all earlier ones could be gone on from as well (`f1`: the furthest
+// edge of any state up to this one), so never more than the true number, and ascending with the distance from where
+// it counts.  A chain of as many dependent steps as the automaton is long; sixteen steps at a time are composed for
+// all states at once, so that what is left in sequence is the chain of every sixteenth place and sixteen steps from
+// each of these side by side (8 lattices of up to 4000 states: 126 us with the whole chain, 29 so).
+constexpr int kHopStates = 7168;  // states of a sequence (kWaveStates)
+constexpr int kHopStride = 16;
+constexpr int kFarHops   = 0x3fffffff;
+__global__ void __launch_bounds__(256) k_hops(const int* __restrict__ state_off, const int* __restrict__ rowptr_f,
+                                              const int* __restrict__ rowptr_b, const uint2* __restrict__ fwd_rec,
+                                              const uint2* __restrict__ bwd_rec, const int* __restrict__ start_l,
+                                              const int* __restrict__ end_l, int* hops_f, int* hops_b,
+                                              fbw_b200_summary* hdr) {
+    typedef cub::BlockScan<int, 256> Scan;
+    __shared__ typename Scan::TempStorage scan;
+    __shared__ unsigned short f1[kHopStates], fa[kHopStates], fb[kHopStates], anchor[kHopStates / kHopStride + 2];
+    __shared__ int notes[2], anchors;
+    if (hdr->error) return;
+    const int  b = blockIdx.x >> 1, tid = threadIdx.x, s0 = state_off[b], Sb = state_off[b + 1] - s0;
+    const bool forward = (blockIdx.x & 1) == 0;
+    // places count from the first state (forward) or the last; the edges that lead on from a state
+    const int*   rowptr = forward ? rowptr_b : rowptr_f;
+    const uint2* rec    = forward ? bwd_rec : fwd_rec;
+    int* hops = forward ? hops_f : hops_b;
+    auto state = [&](int pos) { return s0 + (forward ? pos : Sb - 1 - pos); };
+    if (tid < 2) notes[tid] = 0;
+    __syncthreads();
+    int run = 0, reach = 0, groups = 0;
+    for (int base = 0; base < Sb; base += 256) {
+        const int pos = base + tid;
+        int far = pos;
+        if (pos < Sb) {
+            const int i0 = rowptr[state(pos)], i1 = rowptr[state(pos) + 1];
+            for (int i = i0; i < i1; i++) {
+                const int o = (int)(rec[i].x & 0xffffu), to = forward ? o : Sb - 1 - o;
+                far   = max(far, to);
+                reach = max(reach, to < pos ? 0xffff : to - pos);
+            }
+            groups += max(1, (i1 - i0 + 3) >> 2);
+        }
+        int all;
+        Scan(scan).InclusiveScan(far, far, [](int x, int y) { return max(x, y); }, all);
+        if (pos < min(Sb, kHopStates)) f1[pos] = (unsigned short)min(max(far, run), Sb - 1);
+        run = max(run, all);
+        __syncthreads();
+    }
+    atomicMax(&notes[0], reach);
+    atomicAdd(&notes[1], groups);
+    __syncthreads();
+    if (tid == 0) note_edges(hdr, notes[0], notes[1]);
+    if (Sb > kHopStates || notes[0] == 0xffff) return;  // (no sweep asks for them then)
+    auto twice = [&](const unsigned short* from, unsigned short* to) {
+        for (int pos = tid; pos < Sb; pos += 256) to[pos] = from[from[pos]];
+        __syncthreads();
+    };
+    twice(f1, fa);
+    twice(fa, fb);
+    twice(fb, fa);
+    twice(fa, fb);
+    const int origin = forward ? start_l[b] : Sb - 1 - end_l[b];
+    if (tid == 0) {
+        int n = 0, cur = origin;
+        for (;;) {
+            anchor[n++] = (unsigned short)cur;
+            const int nxt = fb[cur];
+            if (nxt - cur < kHopStride) break;  // the chain ends within the next steps
+            cur = nxt;
+        }
+        anchors = n;
+    }
+    for (int pos = tid; pos <= origin; pos += 256) hops[state(pos)] = 0;
+    __syncthreads();
+    const int n = anchors;
+    for (int j = tid; j < n; j += 256) {
+        int x = anchor[j];
+        for (int i = 1; i <= kHopStride; i++) {
+            const int y = f1[x];
+            for (int pos = x + 1; pos <= y; pos++) hops[state(pos)] = kHopStride * j + i;
+            x = y;
+        }
+    }
+    for (int pos = fb[anchor[n - 1]] + 1 + tid; pos < Sb; pos += 256) hops[state(pos)] = kFarHops;
 }
 
 // single block: everything per sequence that needs the slot counts.  Storage offsets of the run
@@ -947,11 +1048,22 @@ struct RunArgs {
     int fill_ctas;
     int fill_piece;   // floats per bulk store of the background (a multiple of 32, at most kFillFloats)
     int fill_offset;  // where the block of background starts in the sweep CTA's dynamic shared memory (bytes)
+    // Fewest frames from the sequence's start to a state and from a state to its end, at least (left-to-right
+    // automata; see hops_of_sequence)
+    const int *hops_f, *hops_b;
+    // not null: the states that can lie on a path in the frames of a tile, {first, last}, two entries a state from
+    // the sequence's first state (in `carry`, which calls without time chunks do not use)
+    int2* band;
     // not null: the scores as the host has picked them out (fbw_b200_run_with_host with scores in host memory),
     // frame-major like P; k_gather reads them in place of `am`
     const float* picked;
 };
 
+// whether the sweeps leave out states by `band` and k_post can rely on it (a sequence of few states and many frames has
+// no room for the entries)
+__device__ __forceinline__ bool has_band(const RunArgs& a, int Te, int Sb) {
+    return a.band != nullptr && (Te + kTile - 1) / kTile <= 2 * Sb;
+}
 // the raw scores of a sequence
 __device__ __forceinline__ float* raw_scores(const RunArgs& a, int b) { return a.Gf + a.gf_scale * a.gf_off[b]; }
 // The class posteriors of a sequence of Te frames, rows of Dp floats.  Without an array of their own they take
@@ -1471,6 +1583,15 @@ __global__ void __launch_bounds__(32 * kPostWarps, 3) k_post(RunArgs a) {
         const float* __restrict__ Bb = a.Bt + a.ta_off[p.b] + (i64)p.k * p.Sb * kTile + lane;
         float* Gb = a.Gt + a.tg_off[p.b] + (i64)p.k * p.Db * kTile + lane;
         const int4* __restrict__ rec = a.m_rec + p.e0;
+        // states outside [lo, hi] lie on no path of the sequence's length in this tile's frames; the sweeps have left
+        // them out, so their scores are not there
+        int lo = 0, hi = 0xffff;
+        if (has_band(a, p.Te, p.Sb)) {
+            const int2 bd = a.band[2 * (i64)a.state_off[p.b] + p.k];
+            lo = bd.x;
+            hi = bd.y;
+        }
+        auto alive = [&](int4 r) { return (r.x & 0xffff) >= lo && (int)((unsigned)r.x >> 16) <= hi; };
         const bool fold = p.Eb <= kFoldEdges;
         const int i0 = (int)((i64)warp * p.Eb / W), i1 = (int)((i64)(warp + 1) * p.Eb / W);  // this warp's share
 
@@ -1490,9 +1611,10 @@ __global__ void __launch_bounds__(32 * kPostWarps, 3) k_post(RunArgs a) {
                 }
 #pragma unroll
                 for (int j = 0; j < kPostBatch; j++) {
-                    al[j] = Ab[(r[j].x & 0xffff) * kTile];
-                    be[j] = Bb[((unsigned)r[j].x >> 16) * kTile];
-                    g[j]  = Gb[r[j].z * kTile];
+                    const bool on = alive(r[j]);  // uniform
+                    al[j] = on ? Ab[(r[j].x & 0xffff) * kTile] : CUDART_INF_F;
+                    be[j] = on ? Bb[((unsigned)r[j].x >> 16) * kTile] : CUDART_INF_F;
+                    g[j]  = on ? Gb[r[j].z * kTile] : 0.f;
                 }
 #pragma unroll
                 for (int j = 0; j < kPostBatch; j++) {
@@ -1544,10 +1666,11 @@ __global__ void __launch_bounds__(32 * kPostWarps, 3) k_post(RunArgs a) {
             float best = CUDART_INF_F;
             if (p.k * kTile + 1 < p.Te) {
 #pragma unroll 4
-                for (int s = threadIdx.x; s < p.Sb; s += 32 * W) best = fminf(best, A0[s * kTile + 1] + B0[s * kTile]);
+                for (int s = lo + threadIdx.x; s <= min(hi, p.Sb - 1); s += 32 * W) best = fminf(best, A0[s * kTile + 1] + B0[s * kTile]);
             } else {
                 for (int i = threadIdx.x; i < p.Eb; i += 32 * W) {
                     const int4 r = __ldg(rec + i);
+                    if (!alive(r)) continue;
                     best = fminf(best, (A0[(r.x & 0xffff) * kTile] + B0[((unsigned)r.x >> 16) * kTile]) +
                                            (__int_as_float(r.w) + (Gb - lane)[r.z * kTile]));
                 }
@@ -1989,6 +2112,9 @@ void plan_args(RunArgs& a, const void* plan, const fbw_b200_summary& s) {
     a.m_rec    = at<int4>(plan, L.m_rec);
     a.slot_emis = at<int>(plan, L.slot_emis);
     a.order     = at<int>(plan, L.order);
+    a.hops_f    = at<int>(plan, L.hops_f);
+    a.hops_b    = at<int>(plan, L.hops_b);
+    a.band      = nullptr;
     a.T = s.T; a.B = s.B; a.F = s.F;
     a.r0 = 0; a.r1 = (int)s.B;
     a.c_lo = 0; a.c_hi = 1; a.chunk_steps = 1 << 30;
@@ -2105,6 +2231,7 @@ int launch_sweep(const RunArgs& a, int grid, int nt, size_t smem, int smax, int 
 #include "sweep_cluster_b200.inc"
 #include "sweep_scaled_b200.inc"
 #include "sweep_block_b200.inc"
+#include "sweep_wave_b200.inc"
 
 // CTAs per cluster for the sweeps of `items` (sequence, direction) pairs of automata of at most ms
 // states, when `spare` SMs would otherwise stay idle during the call's sweeps.  A cluster spreads the
@@ -2309,6 +2436,8 @@ struct SweepPlan {
     bool clustered;
     bool scaled[FBW_B200_GROUPS];
     bool block[FBW_B200_GROUPS];  // k_sweep_block
+    bool wave[FBW_B200_GROUPS];   // k_sweep_wave
+    bool any_wave;
     int  cs[FBW_B200_GROUPS];
 };
 int base_rank(const fbw_b200_summary& s, int q) { return (int)(((i64)q * s.B) / FBW_B200_GROUPS); }
@@ -2360,16 +2489,21 @@ SweepPlan sweep_plan(const fbw_b200_summary& s) {
         }
         const int items = 2 * (base_rank(s, q0 + per) - base_rank(s, q0));
         // (the background of an output in two steps is written by the sweeps of one CTA)
-        const int cs = p.two_step ? 1 : sweep_cluster_size(gs, items, &spare);
+        // (up to kSmallStates k_sweep_small has a thread for every state; not measured in waves)
+        const int in_waves = !p.two_step && gs > kSmallStates ? wave_cluster_size(s, gs, ge, gd, items, &spare) : 0;
+        const bool wave = in_waves > 0;
+        const int cs = wave ? in_waves : (p.two_step ? 1 : sweep_cluster_size(gs, items, &spare));
+        p.any_wave = p.any_wave || wave;
         // (where the background is written and more sweep CTAs wait than fit two to an SM, the smaller ones of
         // k_sweep_small hold it up less: 256 BPE-CTC sequences 983 against 995 us)
-        const bool block  = cs == 1 && block_shape(s, gs, gd).found && !(p.two_step && s.B > (i64)sm_count());
-        const bool scaled = block || scaled_shape(gs, ge, gd, s.max_degree, cs).found;
+        const bool block  = cs == 1 && !wave && block_shape(s, gs, gd).found && !(p.two_step && s.B > (i64)sm_count());
+        const bool scaled = block || wave || scaled_shape(gs, ge, gd, s.max_degree, cs).found;
         p.clustered = p.clustered || cs > 1;
         for (int q = q0; q < q0 + per; q++) {
             p.cs[q]     = cs;
             p.scaled[q] = scaled;
             p.block[q]  = block;
+            p.wave[q]   = wave;
         }
     }
     return p;
@@ -2378,7 +2512,7 @@ SweepPlan sweep_plan(const fbw_b200_summary& s) {
 // The ranks [r0, r1) as runs of base groups that one sweep launch can serve
 struct SweepRun {
     int  r0, r1, cs;
-    bool scaled, block;
+    bool scaled, block, wave;
     i64  ms, me, md;
 };
 int sweep_runs(const fbw_b200_summary& s, const SweepPlan& p, int r0, int r1, SweepRun* runs) {
@@ -2391,16 +2525,18 @@ int sweep_runs(const fbw_b200_summary& s, const SweepPlan& p, int r0, int r1, Sw
         r.cs = p.cs[q];
         r.scaled = p.scaled[q];
         r.block  = p.block[q];
+        r.wave   = p.wave[q];
         r.ms = s.group_max_states[q];
         r.me = s.group_max_edges[q];
         r.md = s.group_max_slots[q];
-        if (n > 0 && runs[n - 1].cs == r.cs && runs[n - 1].scaled == r.scaled && runs[n - 1].block == r.block) {
+        if (n > 0 && runs[n - 1].cs == r.cs && runs[n - 1].scaled == r.scaled && runs[n - 1].block == r.block && runs[n - 1].wave == r.wave) {
             SweepRun u = runs[n - 1];
             u.r1 = r.r1;
             u.ms = r.ms > u.ms ? r.ms : u.ms;
             u.me = r.me > u.me ? r.me : u.me;
             u.md = r.md > u.md ? r.md : u.md;
-            if (u.block ? block_shape(s, u.ms, u.md).found
+            if (u.wave ? wave_shape(s, u.ms, u.me, u.md, u.cs).found
+                : u.block ? block_shape(s, u.ms, u.md).found
                         : !u.scaled || scaled_shape(u.ms, u.me, u.md, s.max_degree, u.cs).found) {
                 runs[n - 1] = u;
                 continue;
@@ -2431,7 +2567,10 @@ int launch_sweeps(RunArgs a, const SweepRun& r, const fbw_b200_summary& s, cudaS
     const i64 ms = r.ms, me = r.me, md = r.md;
     a.r0 = r.r0;
     a.r1 = r.r1;
-    if (r.block) {
+    if (r.wave) {
+        const int rc = launch_wave(a, wave_shape(s, ms, me, md, cs), 2 * nb, st);
+        if (rc != FBW_B200_OK) return rc;
+    } else if (r.block) {
         const BlockShape bs = block_shape(s, ms, md);
         size_t smem = bs.smem;
         if (a.next_row != nullptr) {  // (as below)
@@ -2515,10 +2654,14 @@ int launch_group(RunArgs a, int r0, int r1, i64 me, const fbw_b200_summary& s, c
     const i64 tiles = (s.max_len + kTile - 1) / kTile;
     SweepRun runs[FBW_B200_GROUPS];
     const int nruns = sweep_runs(s, plan, r0, r1, runs);
+    // (the other sweeps of a batch that has any in waves do not write it: only launches of waves alone rely on it)
+    bool band = plan.any_wave && a.chunk_steps == (1 << 30) && !a.keep_dead_states;
+    for (int i = 0; i < nruns; i++) band = band && runs[i].wave;
+    a.band = band ? reinterpret_cast<int2*>(a.carry) : nullptr;
     if (ev) CUDA_OK(cudaEventRecord(ev[0], st));
     for (int i = 0; (what & kDoGather) && i < nruns; i++) {
         RunArgs g = a;
-        if (!runs[i].scaled || runs[i].cs > 1) g.Gs = nullptr;  // those sweeps read the raw scores
+        if (!runs[i].scaled || runs[i].cs > 1 || runs[i].wave) g.Gs = nullptr;  // those sweeps read the raw scores
         const int rc = launch_gather(g, runs[i].r0, runs[i].r1, runs[i].md, s, st);
         if (rc != FBW_B200_OK) return rc;
     }
@@ -2717,6 +2860,12 @@ static int prepare_impl(const int32_t* edges, const float* weights, const int32_
             at<int>(plan, L.fe), at<int>(plan, L.be), at<int>(plan, L.me), at<int>(plan, L.qpos),
             at<int>(plan, L.edge_off), at<uint2>(plan, L.fwd_rec), at<uint2>(plan, L.bwd_rec),
             at<int4>(plan, L.m_rec), hdr);
+        k_hops<<<2 * (unsigned)B, 256, 0, st>>>(at<int>(plan, L.state_off), at<int>(plan, L.rowptr_f),
+                                                at<int>(plan, L.rowptr_b), at<uint2>(plan, L.fwd_rec),
+                                                at<uint2>(plan, L.bwd_rec), at<int>(plan, L.start_l),
+                                                at<int>(plan, L.end_l), at<int>(plan, L.hops_f),
+                                                at<int>(plan, L.hops_b), hdr);
+        COUNT_LAUNCH(1);
     }
     CUDA_OK(cudaGetLastError());
     return FBW_B200_OK;
