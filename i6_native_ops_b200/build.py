@@ -43,7 +43,7 @@ def build_lib(force: bool = False, verbose: bool = False) -> str:
     # the .inc files are included by fbw_b200.cu; host_fill.cpp is the library's one host-only source
     host_src = os.path.join(csrc, "host_fill.cpp")
     deps = [os.path.join(csrc, f) for f in os.listdir(csrc) if f.endswith((".cu", ".inc"))]
-    deps += [host_src, os.path.join(csrc, "host_fill.h"), os.path.join(csrc, "scaled.h")]
+    deps += [host_src, *(os.path.join(csrc, f) for f in ("host_fill.h", "scaled.h", "sweep_shapes.h"))]
     hdr = os.path.join(INCLUDE, "fbw_b200.h")
     if not force and _newer(LIB, deps + [hdr]):
         return LIB

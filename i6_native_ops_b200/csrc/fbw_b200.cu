@@ -40,6 +40,7 @@
 #include "fbw_b200.h"
 #include "host_fill.h"
 #include "scaled.h"
+#include "sweep_shapes.h"
 
 #include <cuda_runtime.h>
 #include <math_constants.h>

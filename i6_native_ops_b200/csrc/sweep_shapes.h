@@ -1,0 +1,151 @@
+// sweep_shapes.h -- launch shapes of k_sweep_block (sweep_block_b200.inc) and k_sweep_wave (sweep_wave_b200.inc): for
+// which automata they are chosen, threads of each kind, shared memory.  Plain arithmetic on the plan's summary, compiled
+// into the library and, for the tests, by the host compiler alone.
+#pragma once
+#include "fbw_b200.h"
+#include "scaled.h"
+
+#include <stddef.h>
+#include <string.h>
+
+// ---- k_sweep_block ----
+constexpr int kBlockStates = 256;  // threads that compute
+constexpr int kBlockFrames = 8;    // frames of a block
+constexpr int kBlockDegree = 16;   // edges of a state
+constexpr int kBlockRow    = 640;  // classes: the two blocks of score rows are then at most 82 KB
+
+struct BlockDims {
+    int dpmax;                  // row length of the score ring
+    int compute, copy, record;  // threads of each kind (multiples of 32)
+};
+struct BlockSmem {
+    size_t rows, lane, ring, total;
+};
+FBW_HD BlockSmem block_smem(const BlockDims& d) {
+    BlockSmem m;
+    size_t off = 0;
+    m.rows  = off; off += (size_t)16 * kBlockFrames * kBlockStates;
+    m.lane  = off; off += (size_t)4 * kBlockStates;
+    m.ring  = off; off += (size_t)16 * kBlockFrames * d.dpmax;
+    m.total = off;
+    return m;
+}
+
+struct BlockShape {
+    bool      found;
+    int       kreg, nt;
+    bool      split;
+    size_t    smem;
+    BlockDims d;
+};
+// the most groups of three that the edges of a sequence's states take, by target or by source state; 0: not known
+static inline int64_t edge_groups(const fbw_b200_summary& s) { return s.reserved[0] & 0xffffffffll; }
+
+// Launch shape for automata of at most ms states and md class slots
+static inline BlockShape block_shape(const fbw_b200_summary& s, int64_t ms, int64_t md) {
+    BlockShape c;
+    memset(&c, 0, sizeof(c));
+    const int64_t degree = s.max_degree;
+    if (edge_groups(s) == 0 || degree > kBlockDegree || ms > kBlockStates || md > kBlockRow) return c;
+    c.kreg  = degree <= 2 ? 2 : 3;
+    c.split = degree > c.kreg;
+    // a warp may leave as many threads unused as a state has parts less one
+    const int64_t parts = (degree + c.kreg - 1) / c.kreg;
+    const int64_t warps = c.split ? (edge_groups(s) + 32 - parts) / (33 - parts) : (ms + 31) / 32;
+    if (32 * warps > kBlockStates) return c;
+    BlockDims& d = c.d;
+    d.compute = 32 * (int)warps;
+    d.copy    = md > 256 ? 64 : 32;
+    d.record  = d.compute <= 64 ? 32 : 64;
+    // (a launch whose sequences have no edges has no score rows; the steps read a place of the ring all the same, which
+    // has to be there)
+    d.dpmax   = md > 0 ? (int)((md + 3) & ~(int64_t)3) : 4;
+    c.nt    = d.compute + d.copy + d.record;
+    c.smem  = block_smem(d).total;
+    c.found = true;
+    return c;
+}
+
+// ---- k_sweep_wave ----
+constexpr int kWavePiece  = 512;   // threads that compute
+constexpr int kWaveEdges  = 4;     // edges of a thread
+constexpr int kWaveHalo   = 32;    // states before its first one that a piece reads
+constexpr int kWaveBlock  = 4;     // frames of a block
+constexpr int kWaveStates = 7168;  // states of a sequence (hops_of_sequence)
+constexpr int kWaveDegree = 16;    // edges of a state (four parts)
+constexpr int kWaveInbox  = 4;     // blocks kept for the next CTA
+constexpr int kWaveRow    = kWavePiece + kWaveHalo;  // row length of a block's state vectors
+constexpr int kWaveCopy   = 128;   // threads that copy score rows
+constexpr int kWaveRecord = 64;    // threads that record
+
+struct WaveDims {
+    int dpmax;    // row length of the score ring
+    int pieces;   // pieces a CTA can hold
+    int cs;       // CTAs per cluster
+    int split;    // some state has more than kWaveEdges edges
+    int states;   // most states of a sequence
+    int ring;     // blocks of score rows kept: 2, or 1 where two do not fit
+};
+struct WaveSmem {
+    size_t rows, save, lane, inbox, ring, info, total;
+};
+FBW_HD WaveSmem wave_smem(const WaveDims& d) {
+    WaveSmem m;
+    size_t off = 0;
+    m.rows  = off; off += (size_t)16 * kWaveBlock * kWaveRow;
+    m.save  = off; off += (size_t)8 * d.pieces * kWavePiece;
+    m.lane  = off; off += (size_t)4 * d.pieces * kWavePiece;
+    m.inbox = off; off += d.cs > 1 ? (size_t)8 * kWaveInbox * kWaveBlock * kWaveHalo : 0;
+    m.info  = off; off += ((size_t)4 * (4 * d.pieces + 8) + 15) & ~(size_t)15;
+    m.ring  = off;  // (at set-up: row pointers and the first states of the warps)
+    const size_t ring = (size_t)4 * d.ring * kWaveBlock * d.dpmax, setup = (size_t)4 * (d.states + 2) + (size_t)2 * (d.states + 2);
+    off += ring > setup ? ring : setup;
+    m.total = (off + 15) & ~(size_t)15;
+    return m;
+}
+
+struct WaveShape {
+    bool     found;
+    int      pieces;  // of the largest sequence
+    size_t   smem;
+    WaveDims d;
+};
+// Launch shape for automata of at most ms states, me edges and md class slots on clusters of cs CTAs.  What the plan
+// says of the edges: see note_edges.
+static inline WaveShape wave_shape(const fbw_b200_summary& s, int64_t ms, int64_t me, int64_t md, int cs) {
+    WaveShape c;
+    memset(&c, 0, sizeof(c));
+    const int64_t reach = (s.reserved[0] >> 32) & 0xffff, groups = (s.reserved[0] >> 48) & 0xffff;
+    if (groups == 0 || md == 0 || reach > kWaveHalo || s.max_degree > kWaveDegree || ms > kWaveStates) return c;
+    WaveDims& d = c.d;
+    d.cs     = cs;
+    d.split  = s.max_degree > kWaveEdges;
+    d.states = (int)ms;
+    d.dpmax  = (int)((md + 3) & ~(int64_t)3);
+    // warps: a warp may leave as many threads unused as a state has parts less one
+    const int64_t parts = (s.max_degree + kWaveEdges - 1) / kWaveEdges;
+    const int64_t most  = ms + me / kWaveEdges;
+    const int64_t lanes = d.split ? (groups < most ? groups : most) : ms;
+    const int64_t warps = (lanes + 32 - parts) / (33 - parts);
+    c.pieces  = (int)((warps + kWavePiece / 32 - 1) / (kWavePiece / 32));
+    d.pieces  = (c.pieces + cs - 1) / cs;
+    for (d.ring = 2; d.ring >= 1 && !c.found; d.ring--) {
+        c.smem  = wave_smem(d).total;
+        c.found = c.smem <= 227 * 1024 - 256;
+        if (c.found) break;
+    }
+    return c;
+}
+
+// CTAs per cluster for `items` (sequence, direction) pairs: as many as the pieces need to fit, and more, up to one a
+// piece, while SMs would stay idle (see sweep_cluster_size).  0: not for this sweep.
+static inline int wave_cluster_size(const fbw_b200_summary& s, int64_t ms, int64_t me, int64_t md, int items, int* spare) {
+    int least = 1;
+    while (least <= 8 && !wave_shape(s, ms, me, md, least).found) least *= 2;
+    if (least > 8) return 0;
+    const int pieces = wave_shape(s, ms, me, md, least).pieces;
+    int cs = 8;
+    while (cs > least && (cs > pieces || (cs - 1) * items > *spare)) cs >>= 1;
+    *spare -= (cs - 1) * items;
+    return cs;
+}

@@ -1,0 +1,18 @@
+// Host build of the launch shapes of csrc/sweep_shapes.h for sweep_shapes.py.
+#include "sweep_shapes.h"
+
+static fbw_b200_summary summary(int64_t degree, int64_t notes) {
+    fbw_b200_summary s;
+    memset(&s, 0, sizeof(s));
+    s.max_degree  = degree;
+    s.reserved[0] = notes;
+    return s;
+}
+
+// found, registers for edges, split, computing threads, all threads, ring (bytes from the start of shared memory), row
+// length of the ring, shared memory
+extern "C" void block_form(int64_t degree, int64_t notes, int64_t ms, int64_t md, int64_t* out) {
+    const BlockShape c = block_shape(summary(degree, notes), ms, md);
+    const int64_t v[8] = {c.found, c.kreg, c.split, c.d.compute, c.nt, (int64_t)block_smem(c.d).ring, c.d.dpmax, (int64_t)c.smem};
+    memcpy(out, v, sizeof(v));
+}

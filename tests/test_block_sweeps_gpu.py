@@ -96,3 +96,36 @@ def test_time_chunks(cuda, chunks):
                PYTHONPATH=os.pathsep.join([ROOT, os.path.join(ROOT, "tests"), os.environ.get("PYTHONPATH", "")]))
     r = subprocess.run([sys.executable, "-c", CHILD], env=env, capture_output=True, text=True, timeout=600, cwd=ROOT)
     assert r.returncode == 0 and "done" in r.stdout, r.stderr[-2000:]
+
+
+CHILD_NO_EDGES = r"""
+import numpy as np, torch
+import oracle
+from test_automaton_sizes_gpu import on_device
+from test_cluster_sweeps_gpu import check
+from test_block_sweeps_gpu import batch
+from i6_native_ops_b200.fbw import core
+dev = torch.device("cuda:0")
+for deg in (2, 3, 6):
+    am, e, w, se, lens, n = batch(60, deg, 45, 2000)
+    keep = e[3] < 3  # the last sequence: a start, an end, no edge
+    e, w = np.ascontiguousarray(e[:, keep]), w[keep]
+    lens[3] = 40
+    check(core, dev, am, e, w, se, lens, n)
+    want, want_sums = oracle.fbw_oracle(am, e, w, se, lens, n, "f64")
+    lp = np.ascontiguousarray(-am.transpose(1, 0, 2))
+    grad, sums = core.fbw_fused(*on_device(dev, lp, e, w, se, lens), n)
+    assert np.array_equal(sums.cpu().numpy() == 0, want_sums == 0)
+    M = max(1.0, np.abs(want_sums).max())
+    assert np.abs(grad.cpu().numpy().astype(np.float64) + np.exp(-want).transpose(1, 0, 2)).max() <= 8 * M * 2.0 ** -23 + 2e-6
+print("done")
+"""
+
+
+@pytest.mark.parametrize("output", ["expand", "patch"])
+def test_a_launch_without_edges(cuda, output):
+    """Groups of one sequence each, of which the cheapest has no edge; with the background beside the sweeps and without."""
+    env = dict(os.environ, FBW_B200_NUM_GROUPS="4", FBW_B200_OUTPUT=output,
+               PYTHONPATH=os.pathsep.join([ROOT, os.path.join(ROOT, "tests"), os.environ.get("PYTHONPATH", "")]))
+    r = subprocess.run([sys.executable, "-c", CHILD_NO_EDGES], env=env, capture_output=True, text=True, timeout=600, cwd=ROOT)
+    assert r.returncode == 0 and "done" in r.stdout, r.stderr[-2000:]
