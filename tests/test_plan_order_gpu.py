@@ -43,3 +43,22 @@ def test_interleaved_sequences(cuda, S, states, edges):
     d = [torch.from_numpy(np.ascontiguousarray(x)).to(cuda) for x in (am, e.astype(np.int32), w, se.astype(np.int32), lens)]
     got = core.fbw(*d, total, core.DebugOptions())
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("spread", [False, True])
+@pytest.mark.parametrize("total", [65536, 65537, 400001])
+def test_many_state_ids(cuda, total, spread):
+    """Up to 65536 ids k_order looks itself whether they are in order, beyond a launch before it does.  The ids in use
+    come first (in order) or are spread over all (not in order)."""
+    from i6_native_ops_b200.fbw import core
+
+    am, e, w, se, lens, n = batch(90, 3, 40, 30)
+    want = core.fbw(*[torch.from_numpy(x).to(cuda) for x in (am, e, w, se, lens)], n, core.DebugOptions())
+    if spread:
+        new = np.sort(np.random.default_rng(total).permutation(total)[:n])
+        new[-1] = total - 1
+        e = np.stack([new[e[0]], new[e[1]], e[2], e[3]])
+        se = new[se]
+    d = [torch.from_numpy(np.ascontiguousarray(x)).to(cuda) for x in (am, e.astype(np.int32), w, se.astype(np.int32), lens)]
+    got = core.fbw(*d, total, core.DebugOptions())
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
