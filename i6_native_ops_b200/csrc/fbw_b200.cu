@@ -544,7 +544,9 @@ __device__ __forceinline__ void note_edges(fbw_b200_summary* hdr, int reach, int
 // it counts.  A chain of as many dependent steps as the automaton is long; sixteen steps at a time are composed for
 // all states at once, so that what is left in sequence is the chain of every sixteenth place and sixteen steps from
 // each of these side by side (8 lattices of up to 4000 states: 126 us with the whole chain, 29 so).
-constexpr int kHopStates = 7168;  // states of a sequence (kWaveStates)
+// Only k_sweep_wave and what relies on it read the hops and the notes, so nothing of it is done for plans of alignments
+// (`with_sweeps` in prepare_impl), for states of too many edges and for edges that lead too far.
+constexpr int kHopStates = kWaveStates;
 constexpr int kHopStride = 16;
 constexpr int kFarHops   = 0x3fffffff;
 __global__ void __launch_bounds__(256) k_hops(const int* __restrict__ state_off, const int* __restrict__ rowptr_f,
@@ -556,7 +558,7 @@ __global__ void __launch_bounds__(256) k_hops(const int* __restrict__ state_off,
     __shared__ typename Scan::TempStorage scan;
     __shared__ unsigned short f1[kHopStates], fa[kHopStates], fb[kHopStates], anchor[kHopStates / kHopStride + 2];
     __shared__ int notes[2], anchors;
-    if (hdr->error) return;
+    if (hdr->error || hdr->max_degree > kWaveDegree) return;
     const int  b = blockIdx.x >> 1, tid = threadIdx.x, s0 = state_off[b], Sb = state_off[b + 1] - s0;
     const bool forward = (blockIdx.x & 1) == 0;
     // places count from the first state (forward) or the last; the edges that lead on from a state
@@ -589,7 +591,8 @@ __global__ void __launch_bounds__(256) k_hops(const int* __restrict__ state_off,
     atomicAdd(&notes[1], groups);
     __syncthreads();
     if (tid == 0) note_edges(hdr, notes[0], notes[1]);
-    if (Sb > kHopStates || notes[0] == 0xffff) return;  // (no sweep asks for them then)
+    // no sweep asks for the hops then; below, a step of the chain passes at most kWaveHalo states
+    if (Sb > kHopStates || notes[0] > kWaveHalo) return;
     auto twice = [&](const unsigned short* from, unsigned short* to) {
         for (int pos = tid; pos < Sb; pos += 256) to[pos] = from[from[pos]];
         __syncthreads();
@@ -2743,7 +2746,7 @@ size_t fbw_b200_plan_bytes(int64_t B, int64_t E, int64_t S) {
 static int prepare_impl(const int32_t* edges, const float* weights, const int32_t* start_end,
                         const int32_t* seq_lens, int64_t T, int64_t B, int64_t F, int64_t E,
                         int64_t S, void* plan, size_t plan_bytes, fbw_b200_stream_t stream,
-                        bool allow_fast) {
+                        bool allow_fast, bool with_sweeps = true) {
     if (T <= 0 || B <= 0 || F <= 0 || S <= 0 || E < 0) return FBW_B200_BAD_ARGUMENT;
     if (B > 0x7fffffff / 2 || E > 0x7fffffff - 1 || S > 0x7fffffff - 1 || T > 0x7fffffff)
         return FBW_B200_BAD_ARGUMENT;
@@ -2884,12 +2887,14 @@ static int prepare_impl(const int32_t* edges, const float* weights, const int32_
             at<int>(plan, L.fe), at<int>(plan, L.be), at<int>(plan, L.me), at<int>(plan, L.qpos),
             at<int>(plan, L.edge_off), at<uint2>(plan, L.fwd_rec), at<uint2>(plan, L.bwd_rec),
             at<int4>(plan, L.m_rec), hdr);
-        k_hops<<<2 * (unsigned)B, 256, 0, st>>>(at<int>(plan, L.state_off), at<int>(plan, L.rowptr_f),
-                                                at<int>(plan, L.rowptr_b), at<uint2>(plan, L.fwd_rec),
-                                                at<uint2>(plan, L.bwd_rec), at<int>(plan, L.start_l),
-                                                at<int>(plan, L.end_l), at<int>(plan, L.hops_f),
-                                                at<int>(plan, L.hops_b), hdr);
-        COUNT_LAUNCH(1);
+        if (with_sweeps) {
+            k_hops<<<2 * (unsigned)B, 256, 0, st>>>(at<int>(plan, L.state_off), at<int>(plan, L.rowptr_f),
+                                                    at<int>(plan, L.rowptr_b), at<uint2>(plan, L.fwd_rec),
+                                                    at<uint2>(plan, L.bwd_rec), at<int>(plan, L.start_l),
+                                                    at<int>(plan, L.end_l), at<int>(plan, L.hops_f),
+                                                    at<int>(plan, L.hops_b), hdr);
+            COUNT_LAUNCH(1);
+        }
     }
     CUDA_OK(cudaGetLastError());
     return FBW_B200_OK;
@@ -2907,6 +2912,14 @@ int fbw_b200_prepare_general(const int32_t* edges, const float* weights, const i
                              int64_t S, void* plan, size_t plan_bytes, fbw_b200_stream_t stream) {
     return prepare_impl(edges, weights, start_end, seq_lens, T, B, F, E, S, plan, plan_bytes, stream,
                         false);
+}
+
+int fbw_b200_prepare_alignment(const int32_t* edges, const float* weights, const int32_t* start_end,
+                               const int32_t* seq_lens, int64_t T, int64_t B, int64_t F, int64_t E,
+                               int64_t S, int general, void* plan, size_t plan_bytes,
+                               fbw_b200_stream_t stream) {
+    return prepare_impl(edges, weights, start_end, seq_lens, T, B, F, E, S, plan, plan_bytes, stream,
+                        general == 0, false);
 }
 
 int fbw_b200_plan_summary(const void* plan, fbw_b200_summary* summary, fbw_b200_stream_t stream) {

@@ -50,7 +50,7 @@ struct Prepared {
 
 inline Prepared prepare_impl(const torch::Tensor& edges, const torch::Tensor& weights,
                       const torch::Tensor& start_end_states, const torch::Tensor& seq_lens,
-                      int64_t T, int64_t F, int64_t num_states) {
+                      int64_t T, int64_t F, int64_t num_states, bool only_align = false) {
     check_input(edges, torch::kInt32, "edges");
     check_input(weights, torch::kFloat32, "weights");
     check_input(start_end_states, torch::kInt32, "start_end_states");
@@ -73,22 +73,24 @@ inline Prepared prepare_impl(const torch::Tensor& edges, const torch::Tensor& we
     size_t pbytes = fbw_b200_plan_bytes(B, E, num_states);
     Prepared p;
     p.plan = byte_buffer(pbytes, edges.device());
-    check_status(fbw_b200_prepare(edges.data_ptr<int32_t>(), weights.data_ptr<float>(),
-                                  start_end_states.data_ptr<int32_t>(),
-                                  seq_lens.data_ptr<int32_t>(), T, B, F, E, num_states,
-                                  p.plan.data_ptr(), pbytes,
-                                  reinterpret_cast<fbw_b200_stream_t>(stream.stream())));
-    int st = fbw_b200_plan_summary(p.plan.data_ptr(), &p.summary,
-                                   reinterpret_cast<fbw_b200_stream_t>(stream.stream()));
-    if (st == FBW_B200_RETRY_GENERAL) {  // a sequence too large for the fast plan builder
-        check_status(fbw_b200_prepare_general(
-            edges.data_ptr<int32_t>(), weights.data_ptr<float>(),
-            start_end_states.data_ptr<int32_t>(), seq_lens.data_ptr<int32_t>(), T, B, F, E,
-            num_states, p.plan.data_ptr(), pbytes,
-            reinterpret_cast<fbw_b200_stream_t>(stream.stream())));
-        st = fbw_b200_plan_summary(p.plan.data_ptr(), &p.summary,
-                                   reinterpret_cast<fbw_b200_stream_t>(stream.stream()));
-    }
+    auto prepare = [&](bool general) {
+        const int32_t *e = edges.data_ptr<int32_t>(), *se = start_end_states.data_ptr<int32_t>();
+        const int32_t* sl = seq_lens.data_ptr<int32_t>();
+        const float*   w  = weights.data_ptr<float>();
+        auto s = reinterpret_cast<fbw_b200_stream_t>(stream.stream());
+        if (only_align) {
+            check_status(fbw_b200_prepare_alignment(e, w, se, sl, T, B, F, E, num_states, general ? 1 : 0,
+                                                    p.plan.data_ptr(), pbytes, s));
+        } else if (general) {
+            check_status(fbw_b200_prepare_general(e, w, se, sl, T, B, F, E, num_states, p.plan.data_ptr(),
+                                                  pbytes, s));
+        } else {
+            check_status(fbw_b200_prepare(e, w, se, sl, T, B, F, E, num_states, p.plan.data_ptr(), pbytes, s));
+        }
+        return fbw_b200_plan_summary(p.plan.data_ptr(), &p.summary, s);
+    };
+    int st = prepare(false);
+    if (st == FBW_B200_RETRY_GENERAL) st = prepare(true);  // a sequence too large for the fast plan builder
     check_status(st, &p.summary);
     return p;
 }

@@ -45,7 +45,7 @@ std::vector<torch::Tensor> viterbi_impl(const torch::Tensor& scores_in, const to
     auto f32_opts = weights.options();    // float32 on the automata's device
     torch::Tensor alignment = batch_major ? torch::empty({B, T}, int_opts) : torch::empty({T, B}, int_opts);
     torch::Tensor scores    = torch::empty({B}, f32_opts);
-    Prepared p = prepare_impl(edges, weights, start_end_states, seq_lens, T, F, num_states);
+    Prepared p = prepare_impl(edges, weights, start_end_states, seq_lens, T, F, num_states, true);
     auto   stream = at::cuda::getCurrentCUDAStream();
     size_t wbytes = fbw_b200_viterbi_bytes(&p.summary);
     torch::Tensor work = byte_buffer(wbytes, edges.device());

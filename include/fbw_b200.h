@@ -102,6 +102,14 @@ int fbw_b200_prepare_general(const int32_t* edges, const float* weights, const i
                              const int32_t* seq_lens, int64_t T, int64_t B, int64_t F, int64_t E,
                              int64_t S, void* plan, size_t plan_bytes, fbw_b200_stream_t stream);
 
+/* fbw_b200_prepare (general == 0) or fbw_b200_prepare_general (general != 0) for automata that are only
+ * aligned: the same plan without the notes that fbw_b200_run chooses its sweeps of large automata by.  Such a
+ * plan can be run all the same, with other sweeps and so other rounding. */
+int fbw_b200_prepare_alignment(const int32_t* edges, const float* weights, const int32_t* start_end,
+                               const int32_t* seq_lens, int64_t T, int64_t B, int64_t F, int64_t E,
+                               int64_t S, int general, void* plan, size_t plan_bytes,
+                               fbw_b200_stream_t stream);
+
 /* Copy the plan's summary to host memory.  SYNCHRONISES the stream.  Returns
  * FBW_B200_BAD_AUTOMATON if validation failed (summary->error says why), FBW_B200_RETRY_GENERAL if
  * the plan has to be redone with fbw_b200_prepare_general. */
