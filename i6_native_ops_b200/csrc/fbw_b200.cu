@@ -2261,14 +2261,9 @@ int launch_sweep(const RunArgs& a, int grid, int nt, size_t smem, int smax, int 
 // per-frame work of one large sequence over several SMs, which shortens the call only while SMs are
 // free: a call that already has a sweep CTA for every SM gains nothing and pays for the cluster
 // barriers.  Returns 1, 2, 4 or 8 and takes the SMs it uses off `spare`.  FBW_B200_CLUSTER=1|2|4|8 fixes
-// the answer.
+// the answer (also that of wave_cluster_size).
 int sweep_cluster_size(i64 ms, int items, int* spare) {
-    static int forced = -1;
-    if (forced < 0) {
-        const char* e = getenv("FBW_B200_CLUSTER");
-        forced = e ? atoi(e) : 0;
-    }
-    if (forced == 1 || forced == 2 || forced == 4 || forced == 8) return forced;
+    if (forced_cluster_size() > 0) return forced_cluster_size();
     if (ms <= 1024 || items <= 0) return 1;
     // (8 lattice sequences, ms a training step: one CTA 8.6, clusters of two 6.3, of four 5.0, of eight 3.2; 128 lattice
     // sequences, ms a call: 21.6, 19.2, 22.5, 29.6, by this rule 14.6)

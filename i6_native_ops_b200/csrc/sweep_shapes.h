@@ -6,7 +6,18 @@
 #include "scaled.h"
 
 #include <stddef.h>
+#include <stdlib.h>
 #include <string.h>
+
+// CTAs per cluster that FBW_B200_CLUSTER asks for (1, 2, 4 or 8); 0: none
+static inline int forced_cluster_size() {
+    static const int forced = [] {
+        const char* e = getenv("FBW_B200_CLUSTER");
+        const int   n = e ? atoi(e) : 0;
+        return n == 1 || n == 2 || n == 4 || n == 8 ? n : 0;
+    }();
+    return forced;
+}
 
 // ---- k_sweep_block ----
 constexpr int kBlockStates = 256;  // threads that compute
@@ -138,8 +149,10 @@ static inline WaveShape wave_shape(const fbw_b200_summary& s, int64_t ms, int64_
 }
 
 // CTAs per cluster for `items` (sequence, direction) pairs: as many as the pieces need to fit, and more, up to one a
-// piece, while SMs would stay idle (see sweep_cluster_size).  0: not for this sweep.
+// piece, while SMs would stay idle (see sweep_cluster_size); or as many as FBW_B200_CLUSTER says.  0: not for this sweep.
 static inline int wave_cluster_size(const fbw_b200_summary& s, int64_t ms, int64_t me, int64_t md, int items, int* spare) {
+    const int forced = forced_cluster_size();
+    if (forced > 0) return wave_shape(s, ms, me, md, forced).found ? forced : 0;
     int least = 1;
     while (least <= 8 && !wave_shape(s, ms, me, md, least).found) least *= 2;
     if (least > 8) return 0;

@@ -1,5 +1,5 @@
-"""The launch shapes of csrc/sweep_shapes.h, compiled for the host, for batches written down as numpy arrays: which form of
-k_sweep_block a test's batch takes."""
+"""The launch shapes of csrc/sweep_shapes.h, compiled for the host: which form of k_sweep_block or k_sweep_wave a test's
+batch takes."""
 import ctypes
 import functools
 import os
@@ -8,6 +8,7 @@ import tempfile
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 BLOCK_FIELDS = ("found", "kreg", "split", "compute", "threads", "ring", "dpmax", "smem")
+WAVE_FIELDS = ("found", "pieces", "held", "cs", "split", "ring", "smem")
 
 
 @functools.lru_cache(None)
@@ -23,3 +24,23 @@ def block_form(degree, groups, states, slots):
     out = (ctypes.c_int64 * len(BLOCK_FIELDS))()
     lib().block_form(*[ctypes.c_int64(int(x)) for x in (degree, groups, states, slots)], out)
     return dict(zip(BLOCK_FIELDS, out))
+
+
+def wave_notes(reach, groups):
+    """what the general plan notes of edges that lead at most `reach` states on and take `groups` fours"""
+    return reach << 32 | groups << 48
+
+
+def wave_form(degree, reach, groups, states, edges, slots, cs):
+    """the same of k_sweep_wave on clusters of `cs` CTAs, for sequences of at most `edges` edges"""
+    out = (ctypes.c_int64 * len(WAVE_FIELDS))()
+    lib().wave_form(*[ctypes.c_int64(int(x)) for x in (degree, wave_notes(reach, groups), states, edges, slots)], int(cs), out)
+    return dict(zip(WAVE_FIELDS, out))
+
+
+def wave_cluster(degree, reach, groups, states, edges, slots, items, spare):
+    """CTAs per cluster (0: another sweep) and the SMs left of `spare`"""
+    left = ctypes.c_int(spare)
+    cs = lib().wave_cluster(*[ctypes.c_int64(int(x)) for x in (degree, wave_notes(reach, groups), states, edges, slots)],
+                            int(items), ctypes.byref(left))
+    return cs, left.value

@@ -16,3 +16,14 @@ extern "C" void block_form(int64_t degree, int64_t notes, int64_t ms, int64_t md
     const int64_t v[8] = {c.found, c.kreg, c.split, c.d.compute, c.nt, (int64_t)block_smem(c.d).ring, c.d.dpmax, (int64_t)c.smem};
     memcpy(out, v, sizeof(v));
 }
+
+// found, pieces of the largest sequence, pieces a CTA can hold, CTAs a cluster, split, blocks of score rows kept, shared
+// memory
+extern "C" void wave_form(int64_t degree, int64_t notes, int64_t ms, int64_t me, int64_t md, int cs, int64_t* out) {
+    const WaveShape c = wave_shape(summary(degree, notes), ms, me, md, cs);
+    const int64_t v[7] = {c.found, c.pieces, c.d.pieces, c.d.cs, c.d.split, c.d.ring, (int64_t)c.smem};
+    memcpy(out, v, sizeof(v));
+}
+extern "C" int wave_cluster(int64_t degree, int64_t notes, int64_t ms, int64_t me, int64_t md, int items, int* spare) {
+    return wave_cluster_size(summary(degree, notes), ms, me, md, items, spare);
+}
