@@ -2507,10 +2507,17 @@ SweepPlan sweep_plan(const fbw_b200_summary& s) {
         }
         const int items = 2 * (base_rank(s, q0 + per) - base_rank(s, q0));
         // (the background of an output in two steps is written by the sweeps of one CTA)
-        // (up to kSmallStates k_sweep_small has a thread for every state; not measured in waves)
-        const int in_waves = !p.two_step && gs > kSmallStates ? wave_cluster_size(s, gs, ge, gd, items, &spare) : 0;
-        const bool wave = in_waves > 0;
-        const int cs = wave ? in_waves : (p.two_step ? 1 : sweep_cluster_size(gs, items, &spare));
+        // (up to kSmallStates k_sweep_small has a thread for every state: 48 sequences of 600 states and four edges a state
+        // 690 us a call, in waves 1091; 8 of 700 states 486 and 600)
+        const bool may_wave = !p.two_step && gs > kSmallStates && forced_wave() != 0;
+        int spare_other = spare;
+        const int in_waves = may_wave ? wave_clusters(s, gs, ge, gd, items, spare, sm_count()) : 0;
+        const int other    = p.two_step ? 1 : sweep_cluster_size(gs, items, &spare_other);
+        const bool wave = in_waves > 0 && (forced_wave() > 0 || other == 1 || !scaled_shape(gs, ge, gd, s.max_degree, other).found ||
+                                           wave_pays(s, gs, ge, wave_shape(s, gs, ge, gd, in_waves), sm_count()));
+        const int cs = wave ? in_waves : other;
+        if (!wave) spare = spare_other;
+        else if (forced_cluster_size() == 0) spare -= (cs - 1) * items;
         p.any_wave = p.any_wave || wave;
         // (where the background is written and more sweep CTAs wait than fit two to an SM, the smaller ones of
         // k_sweep_small hold it up less: 256 BPE-CTC sequences 983 against 995 us)

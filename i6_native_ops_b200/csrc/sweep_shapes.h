@@ -148,9 +148,46 @@ static inline WaveShape wave_shape(const fbw_b200_summary& s, int64_t ms, int64_
     return c;
 }
 
+// FBW_B200_WAVE=0|1: k_sweep_wave never, wherever it fits; -1: by wave_pays
+static inline int forced_wave() {
+    static const int forced = [] {
+        const char* e = getenv("FBW_B200_WAVE");
+        return e ? atoi(e) : -1;
+    }();
+    return forced;
+}
+// Whether automata that both fit are faster with k_sweep_wave, on clusters of c.d.cs CTAs, than with k_sweep_cluster, in a
+// batch of s.B sequences.  (Where the other sweep would be the one in logarithms, k_sweep, this one is taken in any
+// case: its sums are up to thirty times nearer to the true ones.)
+// k_sweep_cluster meets once a frame, 0.9 to 1.3 us for up to a few hundred states a CTA; k_sweep_wave has a thread for
+// every four edges of a state, 0.8 us a frame for 512 of them and two thirds of it for 512 more, and leaves out what lies
+// on no path.  So it gains where a cluster holds all pieces side by side, where few states have many edges (a warp of the
+// other takes as long as its state with most) and where few frames leave out much; it loses where a CTA holds two pieces
+// of states that all have the same edges.  Measured, us a call with k_sweep_cluster / k_sweep_wave:
+//   some states with far more edges (loops, successors, one or two more; 3.5 on average, the most 9): 24 sequences of 1100
+//     states and 440 frames 928 / 753, 12 of 2500 and 1000: 2906 / 1676, 12 of 3600 and 4320: 13250 / 9485
+//   edges from every state to those 0, 1, 8 and 32 on: 4 sequences of 1100 states and 1320 frames 1303 / 1064 (a piece a CTA),
+//     24: 1771 / 2234, 24 of 1400 and 1680: 2466 / 2897; 12 of 2500 and 3000: 5318 / 4889
+//   0, 1 and 2 on, 24 of 1400 and 700 (no more frames than the way takes): 1509 / 1072
+//   0, 1, 2, 4 and 7 on (two threads a state): 8 of 1100 and 1320: 1823 / 1020 (a piece a CTA), 24: 2157 / 3574; 24 of 1400
+//     and 560: 1103 / 1625; 4 of 2500 and 3000: 3301 / 4093
+static inline bool wave_pays(const fbw_b200_summary& s, int64_t ms, int64_t me, const WaveShape& c, int sms) {
+    const int64_t way = (s.reserved[0] >> 32) & 0xffff, groups = (s.reserved[0] >> 48) & 0xffff;
+    if (4 * s.max_degree * ms >= 7 * me) return true;
+    const bool    one_each = c.pieces <= c.d.cs;
+    const int64_t most     = ms + me / kWaveEdges;
+    if (c.d.split && 2 * (groups < most ? groups : most) > 3 * ms) {  // two threads and more for most states
+        return one_each && 2 * s.B * c.d.cs <= sms;                   // (every CTA of the batch has an SM to itself)
+    }
+    // (the last: a state lies on a path in less than a quarter of the frames)
+    return one_each || ms >= 2048 || 4 * ms >= 3 * way * s.max_len;
+}
+
 // CTAs per cluster for `items` (sequence, direction) pairs: as many as the pieces need to fit, and more, up to one a
-// piece, while SMs would stay idle (see sweep_cluster_size); or as many as FBW_B200_CLUSTER says.  0: not for this sweep.
-static inline int wave_cluster_size(const fbw_b200_summary& s, int64_t ms, int64_t me, int64_t md, int items, int* spare) {
+// piece, while `spare` SMs would stay idle; or as many as FBW_B200_CLUSTER says.  0: they do not fit.
+// Numbers of pieces between the powers of two get the next one where every CTA of the batch has an SM to itself, and the
+// CTAs without a piece leave at once: a second piece costs its CTA two thirds of a frame more.
+static inline int wave_clusters(const fbw_b200_summary& s, int64_t ms, int64_t me, int64_t md, int items, int spare, int sms) {
     const int forced = forced_cluster_size();
     if (forced > 0) return wave_shape(s, ms, me, md, forced).found ? forced : 0;
     int least = 1;
@@ -158,7 +195,7 @@ static inline int wave_cluster_size(const fbw_b200_summary& s, int64_t ms, int64
     if (least > 8) return 0;
     const int pieces = wave_shape(s, ms, me, md, least).pieces;
     int cs = 8;
-    while (cs > least && (cs > pieces || (cs - 1) * items > *spare)) cs >>= 1;
-    *spare -= (cs - 1) * items;
+    auto more_than_needed = [&](int n) { return n > pieces && (n / 2 >= pieces || 2 * s.B * n > sms); };
+    while (cs > least && (more_than_needed(cs) || (cs - 1) * items > spare)) cs >>= 1;
     return cs;
 }

@@ -3,9 +3,7 @@
 states, in edges of the state that has most, in groups of edges, in classes and in how far an edge leads."""
 import numpy as np
 
-from sweep_shapes import block_form, wave_cluster, wave_form
-
-SMS = 148
+from sweep_shapes import block_form, wave_fits, wave_form
 
 
 def automaton(rng, n, hops, ring, classes):
@@ -71,13 +69,13 @@ BLOCK = {
 # of the largest sequence, CTAs a cluster, blocks of score rows kept
 WAVE = {
     "two_whole_pieces": (([1024, 1023, 512], (0, 1, 5, 8), 300, [170, 131, 66], False), (1, 0, 2, 2, 2)),
-    "a_state_more": (([1025, 513, 1024], (0, 1, 5, 8), 300, [171, 70, 130], False), (1, 0, 3, 2, 2)),
-    "a_quarter_off_either_end": (([1300, 1100, 900], (0, 1, 5, 8), 300, [120, 110, 60], True), (1, 0, 3, 2, 2)),
+    "a_state_more": (([1025, 513, 1024], (0, 1, 5, 8), 300, [171, 70, 130], False), (1, 0, 3, 4, 2)),
+    "a_quarter_off_either_end": (([1300, 1100, 900], (0, 1, 5, 8), 300, [120, 110, 60], True), (1, 0, 3, 4, 2)),
     "sixteen_edges_four_parts": (([1100, 900, 40], tuple(range(15)) + (32,), 700, [66, 61, 34], False), (1, 1, 10, 8, 2)),
     "seventeen_edges_and_large": (([1100, 900, 40], tuple(range(16)) + (32,), 700, [66, 61, 34], False), (0, 0, 0, 0, 0)),
-    "one_block_of_rows": (([1500, 1400], (0, 1, 4, 20, 32), 6500, [90, 75], False), (1, 1, 6, 4, 1)),
-    "hardly_any_frames": (([1100, 900, 800], (0, 1, 3, 32), 90, [41, 1, 0], False), (1, 0, 3, 2, 2)),
-    "few_states_many_frames": (([1500, 2, 900], (0, 1, 3, 32), 90, [230, 200, 60], False), (1, 0, 3, 2, 2)),
+    "one_block_of_rows": (([1500, 1400], (0, 1, 4, 20, 32), 6500, [90, 75], False), (1, 1, 6, 8, 1)),
+    "hardly_any_frames": (([1100, 900, 800], (0, 1, 3, 32), 90, [41, 1, 0], False), (1, 0, 3, 4, 2)),
+    "few_states_many_frames": (([1500, 2, 900], (0, 1, 3, 32), 90, [230, 200, 60], False), (1, 0, 3, 4, 2)),
 }
 
 
@@ -98,12 +96,12 @@ def wave_case(name, **kw):
 
 
 def wave_taken(name, cs=None):
-    """by default one launch for the batch (fewer than four sequences, few scores)"""
+    """by default one launch for the batch (fewer than four sequences, few scores), as FBW_B200_WAVE=1 has it"""
     b = wave_case(name)
     d = describe(b[1], b[5])
     args = (d["degree"], d["reach"], d["fours"], d["states"], d["edges"], d["slots"])
     B = len(b[4])
     if cs is None:
-        cs = wave_cluster(*args, items=2 * B, spare=SMS - 2 * B)[0]
+        cs = wave_fits(*args, B, items=2 * B, spare=148 - 2 * B)
     f = wave_form(*args, cs=cs) if cs else wave_form(*args, cs=1)
     return d, (f["found"], f["split"], f["pieces"], f["cs"], f["ring"] if f["found"] else 0)

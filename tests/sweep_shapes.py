@@ -38,9 +38,13 @@ def wave_form(degree, reach, groups, states, edges, slots, cs):
     return dict(zip(WAVE_FIELDS, out))
 
 
-def wave_cluster(degree, reach, groups, states, edges, slots, items, spare):
-    """CTAs per cluster (0: another sweep) and the SMs left of `spare`"""
-    left = ctypes.c_int(spare)
-    cs = lib().wave_cluster(*[ctypes.c_int64(int(x)) for x in (degree, wave_notes(reach, groups), states, edges, slots)],
-                            int(items), ctypes.byref(left))
-    return cs, left.value
+def wave_fits(degree, reach, groups, states, edges, slots, sequences, items, spare, sms=148):
+    """CTAs per cluster with `spare` idle SMs (0: does not fit), in a batch of `sequences`"""
+    return lib().wave_fits(*[ctypes.c_int64(int(x)) for x in (degree, wave_notes(reach, groups), states, edges, slots, sequences)],
+                           int(items), int(spare), int(sms))
+
+
+def wave_is_faster(degree, reach, groups, states, edges, slots, sequences, length, cs, sms=148):
+    """than k_sweep_cluster, in a batch of `sequences` of at most `length` frames, on clusters of `cs` CTAs"""
+    return bool(lib().wave_is_faster(*[ctypes.c_int64(int(x)) for x in (degree, wave_notes(reach, groups), states, edges, slots,
+                                                                        sequences, length)], int(cs), int(sms)))

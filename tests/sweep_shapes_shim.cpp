@@ -24,6 +24,17 @@ extern "C" void wave_form(int64_t degree, int64_t notes, int64_t ms, int64_t me,
     const int64_t v[7] = {c.found, c.pieces, c.d.pieces, c.d.cs, c.d.split, c.d.ring, (int64_t)c.smem};
     memcpy(out, v, sizeof(v));
 }
-extern "C" int wave_cluster(int64_t degree, int64_t notes, int64_t ms, int64_t me, int64_t md, int items, int* spare) {
-    return wave_cluster_size(summary(degree, notes), ms, me, md, items, spare);
+// CTAs per cluster and whether that is faster than k_sweep_cluster, in a batch of so many sequences and so many frames
+extern "C" int wave_fits(int64_t degree, int64_t notes, int64_t ms, int64_t me, int64_t md, int64_t sequences, int items,
+                         int spare, int sms) {
+    fbw_b200_summary s = summary(degree, notes);
+    s.B = sequences;
+    return wave_clusters(s, ms, me, md, items, spare, sms);
+}
+extern "C" int wave_is_faster(int64_t degree, int64_t notes, int64_t ms, int64_t me, int64_t md, int64_t sequences,
+                              int64_t length, int cs, int sms) {
+    fbw_b200_summary s = summary(degree, notes);
+    s.B       = sequences;
+    s.max_len = length;
+    return wave_pays(s, ms, me, wave_shape(s, ms, me, md, cs), sms);
 }
