@@ -14,7 +14,8 @@
 //   k_sweep_small  memory and registers, frames are stepped with one barrier each, next frames' scores
 //               arrive by cp.async; state scores leave several frames at a time (sweep_scaled_b200.inc;
 //               k_sweep_cluster and, in sweep_cluster_b200.inc, k_sweepc on clusters; k_sweep_block for the
-//               smallest automata, sweep_block_b200.inc).
+//               smallest automata, sweep_block_b200.inc, k_sweep_wave for large left-to-right ones,
+//               sweep_wave_b200.inc).
 //   k_post    : per (sequence, 32 frames), lane = frame: edge scores, frame normalisers and class
 //               posteriors, none of which but the posteriors goes through memory.
 //   k_expand  : streams the (T,B,F) output: +inf rows with the few finite posteriors patched in.
@@ -1072,7 +1073,7 @@ struct RunArgs {
     int fill_piece;   // floats per bulk store of the background (a multiple of 32, at most kFillFloats)
     int fill_offset;  // where the block of background starts in the sweep CTA's dynamic shared memory (bytes)
     // Fewest frames from the sequence's start to a state and from a state to its end, at least (left-to-right
-    // automata; see hops_of_sequence)
+    // automata; see k_hops)
     const int *hops_f, *hops_b;
     // not null: the states that can lie on a path in the frames of a tile, {first, last}, two entries a state from
     // the sequence's first state (in `carry`, which calls without time chunks do not use)
@@ -2520,7 +2521,8 @@ SweepPlan sweep_plan(const fbw_b200_summary& s) {
         else if (forced_cluster_size() == 0) spare -= (cs - 1) * items;
         p.any_wave = p.any_wave || wave;
         // (where the background is written and more sweep CTAs wait than fit two to an SM, the smaller ones of
-        // k_sweep_small hold it up less: 256 BPE-CTC sequences 983 against 995 us)
+        // k_sweep_small hold it up less: sequences of 121 states, 400 frames and 10025 classes, us a call with k_sweep_small
+        // and k_sweep_block: 160 641 / 742, 256 1006 / 1004, 400 1609 / 1512)
         const bool block  = cs == 1 && !wave && block_shape(s, gs, gd).found && !(p.two_step && s.B > (i64)sm_count());
         const bool scaled = block || wave || scaled_shape(gs, ge, gd, s.max_degree, cs).found;
         p.clustered = p.clustered || cs > 1;

@@ -82,7 +82,7 @@ constexpr int kWavePiece  = 512;   // threads that compute
 constexpr int kWaveEdges  = 4;     // edges of a thread
 constexpr int kWaveHalo   = 32;    // states before its first one that a piece reads
 constexpr int kWaveBlock  = 4;     // frames of a block
-constexpr int kWaveStates = 7168;  // states of a sequence (hops_of_sequence)
+constexpr int kWaveStates = 7168;  // states of a sequence (k_hops)
 constexpr int kWaveDegree = 16;    // edges of a state (four parts)
 constexpr int kWaveInbox  = 4;     // blocks kept for the next CTA
 constexpr int kWaveRow    = kWavePiece + kWaveHalo;  // row length of a block's state vectors

@@ -192,7 +192,7 @@ int fbw_b200_run_fused(const void* plan, const fbw_b200_summary* summary, const 
  * bit for bit.  A seq_len outside [0, T] (the reference then reads past its table) is treated as 0.
  * batch_major != 0 folds in the wrapper's two transposes (i6_native_ops/fast_viterbi/__init__.py:37,
  * 46): `scores_in` is the caller's (B,T,F) log_probs and `alignment` is written as (B,T).
- * The plan is the one fbw_b200_prepare builds (same automata, same seq_lens); `work` needs
+ * The plan is the one fbw_b200_prepare or fbw_b200_prepare_alignment builds (same automata, same seq_lens); `work` needs
  * fbw_b200_viterbi_bytes(summary) bytes, 256-byte aligned.  Enqueues on `stream`, no synchronisation. */
 size_t fbw_b200_viterbi_bytes(const fbw_b200_summary* summary);
 int fbw_b200_viterbi(const void* plan, const fbw_b200_summary* summary, const float* scores_in,
